@@ -9,6 +9,28 @@
 // also be compiled for the host by the tests.
 #pragma once
 
+// The fits are thousands of instructions of nearly straight code, far more
+// than an SM's instruction caches hold near its warps, so their blocks keep
+// in step: with the warps of a block in the same phase, an instruction is
+// fetched once for all of them.  Every thread of the block takes part in
+// every fit (fitTuples).
+#ifdef __CUDACC__
+#define PG_FIT_PHASE() __syncthreads()
+#else
+#define PG_FIT_PHASE()
+#endif
+
+// Inputs of a block's fits in shared memory, one tuple per thread: hits
+// (3 N doubles) and covariances (6 N floats), each at an odd stride, so that
+// the lanes' accesses fall into different banks.  The fits read them there
+// again where they need them instead of holding them in registers.
+template <int N>
+struct FitTile {
+  static constexpr int kHits = 3 * N, kHitStride = 3 * N | 1;
+  static constexpr int kGe = 6 * N, kGeStride = 6 * N | 1;
+  static constexpr int kBytes = kHitStride * 8 + kGeStride * 4;  // per tuple; the results take 80
+};
+
 __device__ __forceinline__ double sqr(double a) { return a * a; }
 
 template <int R, int C>

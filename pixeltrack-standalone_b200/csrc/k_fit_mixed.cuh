@@ -344,9 +344,9 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
     ccov(2, 1) = I(n, 1);
     ccov(2, 2) = I(n, n);
     ccov = sandwich(J, ccov);
-    translateKarimaki(cpar, ccov, 0.5 * double(emdx), 0.5 * double(emdy));
+    translateKarimaki<false>(cpar, ccov, 0.5 * double(emdx), 0.5 * double(emdy));
     ccov(0, 0) += double((1.f + sqrf(slope)) * multScattF(S[1] - S[0], Bf, ff[2], slope));
-    translateKarimaki(cpar, ccov, double(dx) + x0, double(dy) + y0);
+    translateKarimaki<false>(cpar, ccov, double(dx) + x0, double(dy) + y0);
     cchi2 = 0;
 #pragma unroll
     for (int i = 0; i < n; ++i) {
@@ -381,34 +381,4 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
   out.eta = asinhf(lpar[0]);
   out.chi2 = (cchi2 + lchi2) / float(2 * N - 5);
   (void)B;
-}
-
-// standalone mixed-precision fit of externally supplied tuples
-template <int N>
-__global__ void kBLFitDirectMixed(uint32_t n, const double* hits, const float* hge, double B, float* state,
-                                  float* cov, float* pt, float* eta, float* chi2) {
-  const float Bf = float(B);
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    float H[3 * N];
-    float ge[6 * N];
-    const double* h = hits + size_t(t) * 3 * N;
-    const double x0 = h[0], y0 = h[1];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      H[3 * i + 0] = float(h[3 * i + 0] - x0);
-      H[3 * i + 1] = float(h[3 * i + 1] - y0);
-      H[3 * i + 2] = float(h[3 * i + 2]);
-    }
-#pragma unroll
-    for (int k = 0; k < 6 * N; ++k) ge[k] = hge[size_t(t) * 6 * N + k];
-    FitOut o;
-    blFitMixed<N>(H, ge, x0, y0, Bf, B, o);
-#pragma unroll
-    for (int j = 0; j < 5; ++j) state[size_t(t) * 5 + j] = o.state[j];
-#pragma unroll
-    for (int j = 0; j < 15; ++j) cov[size_t(t) * 15 + j] = o.cov[j];
-    pt[t] = o.pt;
-    eta[t] = o.eta;
-    chi2[t] = o.chi2;
-  }
 }

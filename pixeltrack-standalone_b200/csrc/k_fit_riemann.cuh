@@ -5,7 +5,10 @@
 // TrajectoryStateSoA.h:21-38).  The reference runs it as three kernels with
 // per-fit scratch in global memory; here one thread carries a tuple from
 // the hits to the packed track state, its matrices in registers and local
-// memory.
+// memory.  It is bound by fetching its long code and by local memory; so the
+// covariance blocks go through one piece of code in turn, only their
+// products with the points are kept, and the eigenvectors are chosen by
+// selects (28k -> 19k instructions per 4-hit tuple; 200k tuples: 945 -> 371 us).
 //
 // The smallest eigenvector of the 3x3 Riemann matrix comes from a
 // closed-form solver: eigenvalues from the depressed characteristic cubic
@@ -54,10 +57,9 @@ __device__ __forceinline__ T rfDot(const T* a, const T* b) {
 template <typename T>
 __device__ __forceinline__ void rfOrtho(const T* u, T* e) {
   int ax = 0;
-  if (fabs(u[1]) < fabs(u[ax])) ax = 1;
-  if (fabs(u[2]) < fabs(u[ax])) ax = 2;
-  T a[3] = {T(0), T(0), T(0)};
-  a[ax] = T(1);
+  if (fabs(u[1]) < fabs(u[0])) ax = 1;
+  if (fabs(u[2]) < fabs(ax == 1 ? u[1] : u[0])) ax = 2;
+  const T a[3] = {T(ax == 0), T(ax == 1), T(ax == 2)};
   rfCross(u, a, e);
   const T inv = T(1) / sqrt(rfDot(e, e));
   for (int k = 0; k < 3; ++k) e[k] *= inv;
@@ -65,31 +67,34 @@ __device__ __forceinline__ void rfOrtho(const T* u, T* e) {
 
 // unit null vector of a rank-2 symmetric 3x3 (rows Mx[0..2])
 template <typename T>
-__device__ void rfNull(const T (*Mx)[3], T* v) {
+__device__ __forceinline__ void rfNull(const T (*Mx)[3], T* v) {
   T x[3][3];
   rfCross(Mx[0], Mx[1], x[0]);
   rfCross(Mx[0], Mx[2], x[1]);
   rfCross(Mx[1], Mx[2], x[2]);
   const T n[3] = {rfDot(x[0], x[0]), rfDot(x[1], x[1]), rfDot(x[2], x[2])};
+  // (selects rather than indexed arrays, which would live in local memory)
   int b = 0;
-  if (n[1] > n[b]) b = 1;
-  if (n[2] > n[b]) b = 2;
-  if (n[b] > T(0)) {
-    const T inv = T(1) / sqrt(n[b]);
-    for (int k = 0; k < 3; ++k) v[k] = x[b][k] * inv;
+  if (n[1] > n[0]) b = 1;
+  if (n[2] > (b == 1 ? n[1] : n[0])) b = 2;
+  const T nb = b == 2 ? n[2] : (b == 1 ? n[1] : n[0]);
+  if (nb > T(0)) {
+    const T inv = T(1) / sqrt(nb);
+    for (int k = 0; k < 3; ++k) v[k] = (b == 2 ? x[2][k] : (b == 1 ? x[1][k] : x[0][k])) * inv;
     return;
   }
   const T r[3] = {rfDot(Mx[0], Mx[0]), rfDot(Mx[1], Mx[1]), rfDot(Mx[2], Mx[2])};
   int br = 0;
-  if (r[1] > r[br]) br = 1;
-  if (r[2] > r[br]) br = 2;
-  if (!(r[br] > T(0))) {
+  if (r[1] > r[0]) br = 1;
+  if (r[2] > (br == 1 ? r[1] : r[0])) br = 2;
+  const T rb = br == 2 ? r[2] : (br == 1 ? r[1] : r[0]);
+  if (!(rb > T(0))) {
     v[0] = T(1), v[1] = T(0), v[2] = T(0);
     return;
   }
   T u[3];
-  const T inv = T(1) / sqrt(r[br]);
-  for (int k = 0; k < 3; ++k) u[k] = Mx[br][k] * inv;
+  const T inv = T(1) / sqrt(rb);
+  for (int k = 0; k < 3; ++k) u[k] = (br == 2 ? Mx[2][k] : (br == 1 ? Mx[1][k] : Mx[0][k])) * inv;
   rfOrtho(u, v);
 }
 
@@ -405,152 +410,148 @@ __device__ void rfCircleFit(const double* H, M<2 * N, 2 * N>& V, const S* ff, co
 #pragma unroll
   for (int k = 0; k < n2 * n2; ++k) vsq += V.a[k] * V.a[k];
   const double K = sqr(sqr(s)) * 1. / (4. * q * n) * (2. * vsq + 4. * cmV);
-  // covariances of the centred, scaled points: C[a][b], a <= b
-  M<N, N> Cm[6];  // 00, 01, 02, 11, 12, 22
-  M<N, N> V10;
+  // Covariances of the centred, scaled points: the blocks 00, 01 and 11; the
+  // blocks 02, 12 and 22 follow from them.
+  M<N, N> C00, C01, C11;
 #pragma unroll
   for (int i = 0; i < n; ++i)
 #pragma unroll
     for (int j = 0; j < n; ++j) {
       const int lo = i <= j ? i : j, hi = i <= j ? j : i;
-      Cm[0](i, j) = sqr(s) * V(lo, hi) + K * (mc[lo] * mc[hi]);
-      Cm[1](i, j) = sqr(s) * V(i, j + n) + K * (mc[i] * mc[j + n]);
-      Cm[3](i, j) = sqr(s) * V(lo + n, hi + n) + K * (mc[lo + n] * mc[hi + n]);
-    }
-#pragma unroll
-  for (int i = 0; i < n; ++i)
-#pragma unroll
-    for (int j = 0; j < n; ++j) V10(i, j) = Cm[1](j, i);
-#pragma unroll
-  for (int i = 0; i < n; ++i)
-#pragma unroll
-    for (int j = 0; j < n; ++j) {
-      const double t0 = p3(0, j), t1 = p3(1, j);
-      Cm[2](i, j) = 2. * (Cm[0](i, j) * t0 + Cm[1](i, j) * t1);
-      Cm[4](i, j) = 2. * (V10(i, j) * t0 + Cm[3](i, j) * t1);
-    }
-#pragma unroll
-  for (int i = 0; i < n; ++i)
-#pragma unroll
-    for (int j = i; j < n; ++j) {
-      const double t00 = p3(0, i) * p3(0, j), t01 = p3(0, i) * p3(1, j), t11 = p3(1, i) * p3(1, j);
-      const double t10 = p3(0, j) * p3(1, i);
-      const double a00 = Cm[0](i, j), a01 = Cm[1](i, j), a10 = V10(i, j), a11 = Cm[3](i, j);
-      const double x = 2. * (a00 * a00 + a00 * a01 + a11 * a10 + a11 * a11) +
-                       4. * (a00 * t00 + a01 * t01 + a10 * t10 + a11 * t11);
-      Cm[5](i, j) = x;
-      Cm[5](j, i) = x;
+      C00(i, j) = sqr(s) * V(lo, hi) + K * (mc[lo] * mc[hi]);
+      C01(i, j) = sqr(s) * V(i, j + n) + K * (mc[i] * mc[j + n]);
+      C11(i, j) = sqr(s) * V(lo + n, hi + n) + K * (mc[lo + n] * mc[hi + n]);
     }
   constexpr int nu[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
-  // index of the pair (a, b), a <= b, in Cm / D
-  auto pairIdx = [](int a, int b) { return a == 0 ? b : (a == 1 ? 2 + b : 5); };
-  M<3, 3> C0;
-#pragma unroll
-  for (int p = 0; p < 6; ++p) {
-    const M<N, N>& Cab = Cm[p];
-    double rw[N];
-#pragma unroll
-    for (int j = 0; j < n; ++j) {
-      double t = w[0] * Cab(0, j);
-#pragma unroll
-      for (int i = 1; i < n; ++i) t += w[i] * Cab(i, j);
-      rw[j] = t;
-    }
-    double t = rw[0] * w[0];
-#pragma unroll
-    for (int j = 1; j < n; ++j) t += rw[j] * w[j];
-    C0(nu[p][0], nu[p][1]) = t;
-    C0(nu[p][1], nu[p][0]) = t;
-  }
   M<N, N> Hm;
 #pragma unroll
   for (int i = 0; i < n; ++i)
 #pragma unroll
     for (int j = 0; j < n; ++j) Hm(i, j) = (i == j ? 1. : 0.) - w[j];
   const M<N, 3> sv = mul(Hm, tr(p3));
-  M<N, N> D[6];  // cov(s_v) blocks, a <= b; the others are their transposes
-#pragma unroll
+  // One covariance block C(a, b) after the other: its term of C0 and, with
+  // D(a, b) = cov(s_v)(a, b), the products D(a, b) sv and (its transpose)
+  // D(b, a) sv.  Only those products are kept (27 vectors of N, in local
+  // memory); the loop is not unrolled, so that the block's code, the
+  // largest of the fit, is fetched once.
+  double C0v[6], DS[3][3][3][N];  // DS[a][b][col]
+#pragma unroll 1
   for (int p = 0; p < 6; ++p) {
-    const M<N, N> t = mul(mul(Hm, Cm[p]), tr(Hm));
+    M<N, N> Cab;
 #pragma unroll
     for (int i = 0; i < n; ++i)
 #pragma unroll
-      for (int j = 0; j < n; ++j) D[p](i, j) = t(i, j) * (w[i] * w[j]);
-  }
-  auto Dat = [&](int a, int b, int r, int m) {
-    return a <= b ? D[pairIdx(a, b)](r, m) : D[pairIdx(b, a)](m, r);
-  };
-  auto mv = [&](int a, int b, int col, bool twice, double* out) {
+      for (int j = 0; j < n; ++j) {
+        const double t0 = p3(0, j), t1 = p3(1, j);
+        if (p == 0) {
+          Cab(i, j) = C00(i, j);
+        } else if (p == 1) {
+          Cab(i, j) = C01(i, j);
+        } else if (p == 2) {
+          Cab(i, j) = 2. * (C00(i, j) * t0 + C01(i, j) * t1);
+        } else if (p == 3) {
+          Cab(i, j) = C11(i, j);
+        } else if (p == 4) {
+          Cab(i, j) = 2. * (C01(j, i) * t0 + C11(i, j) * t1);
+        } else if (i <= j) {
+          const double t00 = p3(0, i) * t0, t01 = p3(0, i) * t1, t11 = p3(1, i) * t1, t10 = t0 * p3(1, i);
+          const double a00 = C00(i, j), a01 = C01(i, j), a10 = C01(j, i), a11 = C11(i, j);
+          Cab(i, j) = 2. * (a00 * a00 + a00 * a01 + a11 * a10 + a11 * a11) +
+                      4. * (a00 * t00 + a01 * t01 + a10 * t10 + a11 * t11);
+        }
+      }
+    if (p == 5) {
 #pragma unroll
-    for (int r = 0; r < n; ++r) {
-      double t = (twice ? 2. * Dat(a, b, r, 0) : Dat(a, b, r, 0)) * sv(0, col);
+      for (int i = 1; i < n; ++i)
 #pragma unroll
-      for (int m = 1; m < n; ++m) t += (twice ? 2. * Dat(a, b, r, m) : Dat(a, b, r, m)) * sv(m, col);
-      out[r] = t;
+        for (int j = 0; j < i; ++j) Cab(i, j) = Cab(j, i);
     }
-  };
-  auto dotc = [&](int col, const double* x) {
-    double t = sv(0, col) * x[0];
+    {
+      double rw[N];
 #pragma unroll
-    for (int r = 1; r < n; ++r) t += sv(r, col) * x[r];
-    return t;
-  };
+      for (int j = 0; j < n; ++j) {
+        double t = w[0] * Cab(0, j);
+#pragma unroll
+        for (int i = 1; i < n; ++i) t += w[i] * Cab(i, j);
+        rw[j] = t;
+      }
+      double t = rw[0] * w[0];
+#pragma unroll
+      for (int j = 1; j < n; ++j) t += rw[j] * w[j];
+      C0v[p] = t;
+    }
+    M<N, N> D = mul(mul(Hm, Cab), tr(Hm));
+#pragma unroll
+    for (int i = 0; i < n; ++i)
+#pragma unroll
+      for (int j = 0; j < n; ++j) D(i, j) = D(i, j) * (w[i] * w[j]);
+    const int a = nu[p][0], b = nu[p][1];
+#pragma unroll
+    for (int col = 0; col < 3; ++col) {
+#pragma unroll
+      for (int r = 0; r < n; ++r) {
+        double t = D(0, r) * sv(0, col), u = D(r, 0) * sv(0, col);
+#pragma unroll
+        for (int m = 1; m < n; ++m) {
+          t += D(m, r) * sv(m, col);
+          u += D(r, m) * sv(m, col);
+        }
+        DS[b][a][col][r] = t;  // overwritten by the next line on the diagonal
+        DS[a][b][col][r] = u;
+      }
+    }
+  }
+  M<3, 3> C0;
+#pragma unroll
+  for (int p = 0; p < 6; ++p) {
+    C0(nu[p][0], nu[p][1]) = C0v[p];
+    C0(nu[p][1], nu[p][0]) = C0v[p];
+  }
+  // The covariance of A's elements: with g(x, i, (k, l)) =
+  // sv_i . (D(x, l) sv_k + D(x, k) sv_l), E((i, j), (k, l)) = g(j, i) + g(i, j);
+  // for i = j, and inside g for k = l, the two equal terms are one term
+  // doubled, which is exact.
   M<6, 6> E;
-#pragma unroll 1
-  for (int a = 0; a < 6; ++a) {
-    const int i = nu[a][0], j = nu[a][1];
-#pragma unroll 1
-    for (int b = a; b < 6; ++b) {
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+#pragma unroll
+    for (int b = 0; b < 6; ++b) {
       const int k = nu[b][0], l = nu[b][1];
-      double t0[N], t1[N], u[N], z[N];
-      if (l == k) {
-        mv(j, l, l, true, t0);
-        if (i == j) {
+      double t0[N];
 #pragma unroll
-          for (int r = 0; r < n; ++r) t1[r] = t0[r];
-        } else {
-          mv(i, l, l, true, t1);
-        }
-      } else {
-        mv(j, l, k, false, u);
-        mv(j, k, l, false, z);
+      for (int r = 0; r < n; ++r)
+        t0[r] = l == k ? 2. * DS[x][l][l][r] : DS[x][l][k][r] + DS[x][k][l][r];
 #pragma unroll
-        for (int r = 0; r < n; ++r) t0[r] = u[r] + z[r];
-        if (i == j) {
+      for (int i = 0; i < 3; ++i) {
+        const int a = i < x ? (i == 0 ? x : 2 + x) : (x == 0 ? i : (x == 1 ? 2 + i : 5));  // the pair of i and x
+        if (b < a) continue;
+        double t = sv(0, i) * t0[0];
 #pragma unroll
-          for (int r = 0; r < n; ++r) t1[r] = t0[r];
-        } else {
-          mv(i, l, k, false, u);
-          mv(i, k, l, false, z);
-#pragma unroll
-          for (int r = 0; r < n; ++r) t1[r] = u[r] + z[r];
-        }
+        for (int r = 1; r < n; ++r) t += sv(r, i) * t0[r];
+        E(a, b) = i == x ? 2. * t : (i > x ? t : E(a, b) + t);
       }
-      double e;
-      if (i == j) {
-        double tt[N];
-#pragma unroll
-        for (int r = 0; r < n; ++r) tt[r] = t0[r] + t1[r];
-        e = 0. + dotc(i, tt);
-      } else {
-        e = 0. + (dotc(i, t0) + dotc(j, t1));
-      }
-      E(a, b) = e;
-      E(b, a) = e;
     }
   }
+#pragma unroll
+  for (int a = 0; a < 6; ++a)
+#pragma unroll
+    for (int b = 0; b < a; ++b) E(a, b) = E(b, a);
   M<3, 6> J2;  // numerical Jacobian of the smallest eigenvector
 #pragma unroll 1
   for (int a = 0; a < 6; ++a) {
     const int i = nu[a][0], j = nu[a][1];
-    const double dl = fabs(A(i, j) * kRfDeriv);
+    double aij = 0.;  // A(i, j)
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int m = r; m < 3; ++m) aij = r == i && m == j ? A(r, m) : aij;
+    const double dl = fabs(aij * kRfDeriv);
     double ad[3][3];
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int m = 0; m < 3; ++m) ad[r][m] = A(r, m);
-    ad[i][j] = A(i, j) + dl;
-    if (j != i) ad[j][i] = A(j, i) + dl;
+      for (int m = 0; m < 3; ++m)
+        ad[r][m] = (r == i && m == j) || (r == j && m == i) ? A(r, m) + dl : A(r, m);
     double vf[3];
     if constexpr (std::is_same<S, float>::value) {
       // the single-precision solve of the reference, natively
@@ -649,11 +650,6 @@ __device__ void rfLineFit(const double* H, const float* ge, const RfCircle& circ
   M<2, 2> rot;
   rot(0, 0) = sn, rot(0, 1) = cs, rot(1, 0) = -cs, rot(1, 1) = sn;
   const double o0 = circle.par[0], o1 = circle.par[1];
-  M<6, 6> Cov = rfZero<6, 6>();
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) Cov(a, b) = circle.cov(a, b);
   double szz[N], sArcD[N];  // cov_sz(1,1) and the arc length per hit
   S sArc[N], zz[N];
 #pragma unroll
@@ -674,21 +670,24 @@ __device__ void rfLineFit(const double* H, const float* ge, const RfCircle& circ
     }
     sArc[i] = S(sArcD[i]);
     const S temp0 = S(-circle.q) * S(circle.par[2]) * S(1) / (dot * dot + cross * cross);
-    M<2, 6> Jx = rfZero<2, 6>();
-    Jx(0, 0) = -temp0 * ((py + so1) * dot - (px - so0) * cross);
-    Jx(0, 1) = temp0 * ((px + so0) * dot - (so1 - py) * cross);
-    Jx(0, 2) = at;
-    Jx(0, 3) = temp0 * (so1 * dot + so0 * cross);
-    Jx(0, 4) = temp0 * (-so0 * dot + so1 * cross);
-    Jx(1, 5) = 1.;
+    const double j0 = -temp0 * ((py + so1) * dot - (px - so0) * cross);
+    const double j1 = temp0 * ((px + so0) * dot - (so1 - py) * cross);
+    const double j2 = at;
+    const double j3 = temp0 * (so1 * dot + so0 * cross);
+    const double j4 = temp0 * (-so0 * dot + so1 * cross);
+    // J Cov J^T without its zero terms: J's rows are (j0..j4, 0) and
+    // (0, .., 0, 1), Cov holds the circle's and the hit's 3x3 blocks
     const float* g = ge + 6 * i;
-    Cov(3, 3) = g[0];
-    Cov(4, 4) = g[2];
-    Cov(5, 5) = g[5];
-    Cov(3, 4) = Cov(4, 3) = g[1];
-    Cov(3, 5) = Cov(5, 3) = g[3];
-    Cov(4, 5) = Cov(5, 4) = g[4];
-    const M<2, 2> t = sandwich(Jx, Cov);
+    const double gxx = g[0], gxy = g[1], gyy = g[2], gxz = g[3], gyz = g[4], gzz = g[5];
+    double m0[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) m0[k] = j0 * circle.cov(0, k) + j1 * circle.cov(1, k) + j2 * circle.cov(2, k);
+    const double m3 = j3 * gxx + j4 * gxy, m4 = j3 * gxy + j4 * gyy, m5 = j3 * gxz + j4 * gyz;
+    M<2, 2> t;
+    t(0, 0) = m0[0] * j0 + m0[1] * j1 + m0[2] * j2 + m3 * j3 + m4 * j4;
+    t(0, 1) = m5;
+    t(1, 0) = gxz * j3 + gyz * j4;
+    t(1, 1) = gzz;
     szz[i] = sandwich(rot, t)(1, 1);
     zz[i] = S(H[3 * i + 2]);
   }
@@ -824,28 +823,4 @@ __device__ void rfFit(const double* H, const float* ge, double B, FitOut& o) {
   o.pt = float(B / fabs(circle.par[2]));
   o.eta = asinhf(float(line.par[0]));
   o.chi2 = float((circle.chi2 + line.chi2) / (2 * N - 5));
-}
-
-// standalone Riemann fit of externally supplied tuples
-template <int N, typename S>
-__global__ void __launch_bounds__(128) kRiemannFitDirect(uint32_t n, const double* hits, const float* hge, double B,
-                                                         float* state, float* cov, float* pt, float* eta,
-                                                         float* chi2) {
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    double H[3 * N];
-    float ge[6 * N];
-#pragma unroll
-    for (int k = 0; k < 3 * N; ++k) H[k] = hits[size_t(t) * 3 * N + k];
-#pragma unroll
-    for (int k = 0; k < 6 * N; ++k) ge[k] = hge[size_t(t) * 6 * N + k];
-    FitOut o;
-    rfFit<N, S>(H, ge, B, o);
-#pragma unroll
-    for (int j = 0; j < 5; ++j) state[size_t(t) * 5 + j] = o.state[j];
-#pragma unroll
-    for (int j = 0; j < 15; ++j) cov[size_t(t) * 15 + j] = o.cov[j];
-    pt[t] = o.pt;
-    eta[t] = o.eta;
-    chi2[t] = o.chi2;
-  }
 }
