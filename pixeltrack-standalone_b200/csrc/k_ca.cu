@@ -1241,12 +1241,22 @@ __global__ void kTupleDet(Workspace ws) {
 // places the bins, and fills them in ascending tuple order (the serial fill
 // order) with one scan of the three counters packed into 64 bits, so that
 // the content stays deterministic when a bin overflows.
+constexpr uint32_t kMultiplicityCtas = 8;  // in a small batch; pairs in a large one
+// A cluster of P CTAs per event splits the tuples (CTA r takes the r-th part,
+// its counts read by the others through distributed shared memory), since
+// one CTA's two walks are bound by the latency of its loads: 12 uneven events
+// (PU 20-200) took 427 us, all of it the heaviest event's.
 __global__ void __launch_bounds__(1024) kMultiplicity(Workspace ws) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
   __shared__ uint32_t cnt[8], start[8];
   __shared__ uint64_t scanSh[33];
-  const uint32_t e = blockIdx.x;
+  __shared__ uint64_t sTot;  // this CTA's three counts, 20 bits each
+  const uint32_t rank = cl.block_rank(), P = cl.num_blocks();
+  const uint32_t e = blockIdx.y;
   EventCounters* c = ws.ev + e;
-  const uint32_t nt = c->nTuples;
+  const uint32_t all = c->nTuples;
+  const uint32_t first = uint32_t(uint64_t(all) * rank / P), nt = uint32_t(uint64_t(all) * (rank + 1) / P);
   const uint32_t* toff = ws.tupleOff + size_t(e) * (ws.cap.tuples + 1);
   const uint8_t* q = ws.quality + size_t(e) * ws.cap.tuples;
   uint32_t* tm = ws.tmOff + size_t(e) * 16;
@@ -1260,8 +1270,8 @@ __global__ void __launch_bounds__(1024) kMultiplicity(Workspace ws) {
   // each of its tuples as a 2-bit code (up to 128 steps), so the second walk,
   // which places the tuples, needs no loads.
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t R = (nt + nw * 32 - 1) / (nw * 32) * 32;
-  const uint32_t w0 = min(nt, warp * R), w1 = min(nt, w0 + R);
+  const uint32_t R = (nt - first + nw * 32 - 1) / (nw * 32) * 32;
+  const uint32_t w0 = min(nt, first + warp * R), w1 = min(nt, w0 + R);
   const uint32_t steps = (w1 - w0 + 31) / 32;
   constexpr uint32_t kKeptSteps = 128;
   const bool kept = steps <= kKeptSteps;
@@ -1292,23 +1302,34 @@ __global__ void __launch_bounds__(1024) kMultiplicity(Workspace ws) {
   n5 = __reduce_add_sync(0xffffffffu, n5);
   uint64_t tot;
   const uint64_t mine = uint64_t(n3) | (uint64_t(n4) << 20) | (uint64_t(n5) << 40);
-  const uint64_t warpPre = __shfl_sync(0xffffffffu, blockExclusiveScan64(lane == 0 ? mine : 0ull, scanSh, &tot), 0);
+  uint64_t warpPre = __shfl_sync(0xffffffffu, blockExclusiveScan64(lane == 0 ? mine : 0ull, scanSh, &tot), 0);
+  if (threadIdx.x == 0) sTot = tot;
+  cl.sync();
+  tot = 0;
+  for (uint32_t r = 0; r < P; ++r) {
+    const uint64_t t = *cl.map_shared_rank(&sTot, r);
+    if (r < rank) warpPre += t;
+    tot += t;
+  }
+  cl.sync();  // no CTA ends while another reads its count
   if (threadIdx.x == 0) {
     for (int b = 0; b < 8; ++b) cnt[b] = (b >= 3 && b <= 5) ? uint32_t((tot >> (20 * (b - 3))) & 0xfffffu) : 0u;
     uint32_t acc = 0;
     for (int b = 0; b < 8; ++b) {
       start[b] = acc;
-      tm[8 + b] = acc;  // start of bin b
-      tm[b] = cnt[b];
-      if (cnt[b] > ws.cap.multiplicity) c->flags |= kFlagFitBinOverflow;
+      if (rank == 0) {
+        tm[8 + b] = acc;  // start of bin b
+        tm[b] = cnt[b];
+        if (cnt[b] > ws.cap.multiplicity) c->flags |= kFlagFitBinOverflow;
+      }
       acc += cnt[b];
     }
-    if (acc > ws.cap.multiplicity) c->flags |= kFlagTmOverflow;
+    if (rank == 0 && acc > ws.cap.multiplicity) c->flags |= kFlagTmOverflow;
     // the neighbour and track list pools of the reference (CellNeighborsVector,
     // CellTracksVector: cap.lists lists including the reserved empty one);
     // beyond them its lists depend on the order the cells are visited
-    if (c->nNbrLists > ws.cap.lists) c->flags |= kFlagNbrPoolOverflow;
-    if (c->nTrkLists > ws.cap.lists) c->flags |= kFlagTrkPoolOverflow;
+    if (rank == 0 && c->nNbrLists > ws.cap.lists) c->flags |= kFlagNbrPoolOverflow;
+    if (rank == 0 && c->nTrkLists > ws.cap.lists) c->flags |= kFlagTrkPoolOverflow;
   }
   __syncthreads();
   // the serial fill order: ascending tuple index (warps in range order, then
@@ -1693,7 +1714,11 @@ cudaError_t runCA(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStrea
   PG_PROBED("kEarlyDup", stream, kEarlyDup<<<dim3(tunedGrid(ws, kTuneEarlyDup, gx), nEvents), 256, 0, stream>>>(ws));
   PG_PROBED("kTupleDet", stream, kTupleDet<<<dim3(tunedGrid(ws, kTuneTupleDet, gx), nEvents), 256, 0, stream>>>(ws));
   // ---- tuple multiplicity for the fits
-  PG_PROBED("kMultiplicity", stream, kMultiplicity<<<nEvents, 1024, 0, stream>>>(ws));
+  cudaError_t le = cudaSuccess;
+  PG_PROBED("kMultiplicity", stream,
+            le = launchClustered(kMultiplicity, nEvents <= kClusterMaxEvents ? kMultiplicityCtas : 2u, nEvents, 1024, 0,
+                                 stream, ws));
+  if (le != cudaSuccess) return le;
   // ---- late fishbone (CAHitNtupletGeneratorKernels.cc:133-136)
   if (ws.ca.lateFishbone)
     PG_PROBED("kFishbone", stream, kFishbone<<<dim3(tunedGrid(ws, kTuneFishbone, gx * 2), nEvents), 256, 0, stream>>>(ws, true));
