@@ -36,7 +36,7 @@ constexpr size_t kTrackBytes = 9 * 4 + 2 + 2;
 constexpr size_t kVtxSmemBytes = kSmemTracks * kTrackBytes;
 // with the kernel's static shared memory (about 9.4 KB) within the 227 KB of a block
 static_assert(kVtxSmemBytes + 10 * 1024 <= 227 * 1024, "vertex shared memory");
-constexpr uint32_t kVtxCtas = 4;  // CTAs per event in a small batch
+constexpr uint32_t kVtxCtas = 8;  // CTAs per event in a small batch
 
 struct VtxScratch {
   float *zt, *ezt2, *ptt2, *zz;
@@ -87,120 +87,144 @@ __device__ __forceinline__ VtxScratch scratchOf(const Workspace& ws, uint32_t e)
   return s;
 }
 
-// group tracks by vertex id (ascending track order inside each vertex)
-__device__ void groupByVertex(const VtxScratch& s, uint32_t nt, uint32_t nv, uint32_t* vOff, uint32_t* vCur,
-                              uint32_t* scanSh) {
-  for (uint32_t v = threadIdx.x; v <= nv; v += blockDim.x) {
-    vOff[v] = 0;
-    vCur[v] = 0;
-  }
+// Groups n items by key in item order (a stable counting sort): off[0..nb]
+// receives the groups' starts, place(i, pos) every item with a key < nb.
+// Each of W warps walks a contiguous part of the items twice, first counting
+// its keys in its own row of tab (nb entries), then, after the rows' prefix
+// sums, placing them; lanes of the same key are ranked among themselves (a
+// ballot per key bit: a match instruction costs more than the ten ballots of
+// the largest key).  So a warp walks n / W items, where letting each warp own a range
+// of keys made every warp walk all of them (1087 tracks: 21k of the kernel's
+// 113k cycles for the z histogram and 12k for each grouping by vertex).
+// Called by the whole block; ends with a barrier.
+template <typename Key, typename Place>
+__device__ __forceinline__ void orderedFill(uint32_t n, uint32_t nb, uint16_t* tab, uint32_t W, uint32_t* off,
+                                            uint32_t* scanSh, Key&& key, Place&& place) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t k = threadIdx.x; k < nb * W; k += blockDim.x) tab[k] = 0;
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
-    int32_t v = s.iv[i];
-    if (v >= 0 && uint32_t(v) < nv) atomicAdd(&vOff[v], 1u);
+  const uint32_t part = (n + W * 32 - 1) / (W * 32) * 32;
+  const uint32_t i0 = warp < W ? min(n, warp * part) : n, i1 = min(n, i0 + part);
+  uint16_t* row = tab + warp * nb;
+  const uint32_t bits = 32 - __clz(nb | 1);
+  auto sameKey = [&](uint32_t b) {
+    uint32_t m = __ballot_sync(0xffffffffu, b < nb);
+    for (uint32_t k = 0; k < bits; ++k) {
+      const bool one = (b >> k) & 1u;
+      const uint32_t with = __ballot_sync(0xffffffffu, one);
+      m &= one ? with : ~with;
+    }
+    return m;  // meaningless for lanes without a key below nb
+  };
+  for (uint32_t ib = i0; ib < i1; ib += 32) {
+    const uint32_t i = ib + lane, b = i < i1 ? key(i) : 0xffffffffu;
+    const uint32_t peers = sameKey(b);
+    if (b < nb && (peers & lanemaskLt()) == 0) row[b] = uint16_t(row[b] + __popc(peers));
+    __syncwarp();
   }
   __syncthreads();
   uint32_t carry = 0;
-  for (uint32_t v0 = 0; v0 <= nv; v0 += blockDim.x) {
-    uint32_t v = v0 + threadIdx.x;
-    uint32_t c = v <= nv ? vOff[v] : 0u;
+  for (uint32_t b0 = 0; b0 <= nb; b0 += blockDim.x) {
+    const uint32_t b = b0 + threadIdx.x;
+    uint32_t run = 0;
+    if (b < nb) {
+#pragma unroll 8
+      for (uint32_t w = 0; w < W; ++w) {
+        const uint32_t t = tab[w * nb + b];
+        tab[w * nb + b] = uint16_t(run);
+        run += t;
+      }
+    }
     uint32_t tot;
-    uint32_t pre = blockExclusiveScan(c, scanSh, &tot);
-    if (v <= nv) vOff[v] = carry + pre;
+    const uint32_t pre = blockExclusiveScan(run, scanSh, &tot);
+    if (b <= nb) off[b] = carry + pre;
     carry += tot;
   }
   __syncthreads();
-  // ordered fill (ascending track order inside each vertex).  Few vertices:
-  // one warp per vertex walks the tracks, 128 at a time, until it has found
-  // them all.  Many: warp w owns a range of vertices and walks the tracks
-  // once, 32 at a time; lanes of the same vertex are ranked among themselves
-  // (match) and its cursor (vCur) advances by their number.
-  const uint32_t lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if (nv <= 2 * nw) {
-    for (uint32_t v = threadIdx.x >> 5; v < nv; v += nw) {
-      uint32_t pos = vOff[v];
-      const uint32_t end = vOff[v + 1];
-      for (uint32_t i0 = 0; i0 < nt && pos < end; i0 += 128) {
-        bool in[4];
-#pragma unroll
-        for (uint32_t u = 0; u < 4; ++u) {
-          const uint32_t i = i0 + u * 32 + lane;
-          in[u] = i < nt && s.iv[i] == int32_t(v);
-        }
-#pragma unroll
-        for (uint32_t u = 0; u < 4; ++u) {
-          const uint32_t m = __ballot_sync(0xffffffffu, in[u]);
-          if (in[u]) s.list[pos + __popc(m & lanemaskLt())] = i0 + u * 32 + lane;
-          pos += __popc(m);
-        }
-      }
+  for (uint32_t ib = i0; ib < i1; ib += 32) {
+    const uint32_t i = ib + lane, b = i < i1 ? key(i) : 0xffffffffu;
+    const uint32_t peers = sameKey(b);
+    if (b < nb) {
+      const uint32_t at = row[b];
+      place(i, off[b] + at + __popc(peers & lanemaskLt()));
+      __syncwarp(peers);
+      if ((peers & lanemaskLt()) == 0) row[b] = uint16_t(at + __popc(peers));
     }
-  } else {
-    for (uint32_t v = threadIdx.x; v < nv; v += blockDim.x) vCur[v] = vOff[v];
-    __syncthreads();
-    const uint32_t vpw = (nv + nw - 1) / nw, vLo = (threadIdx.x >> 5) * vpw, vHi = min(nv, vLo + vpw);
-    for (uint32_t i0 = 0; i0 < nt && vLo < vHi; i0 += 32) {
-      const uint32_t i = i0 + lane;
-      const int32_t v = i < nt ? s.iv[i] : -1;
-      const bool in = v >= int32_t(vLo) && v < int32_t(vHi);
-      const uint32_t m = __ballot_sync(0xffffffffu, in);
-      if (m) {
-        const uint32_t peers = __match_any_sync(0xffffffffu, in ? uint32_t(v) : 0xffffffffu) & m;
-        if (in) {
-          s.list[vCur[v] + __popc(peers & lanemaskLt())] = i;
-          __syncwarp(peers);
-          if ((peers & lanemaskLt()) == 0) vCur[v] += __popc(peers);
-        }
-        __syncwarp();
-      }
-    }
+    __syncwarp();
   }
   __syncthreads();
 }
 
+// group tracks by vertex id (ascending track order inside each vertex);
+// tab: tabBytes of shared memory
+__device__ void groupByVertex(const VtxScratch& s, uint32_t nt, uint32_t nv, uint32_t* vOff, uint32_t* scanSh,
+                              uint16_t* tab, uint32_t tabBytes) {
+  const uint32_t W = min(blockDim.x >> 5, tabBytes / 2 / max(nv, 1u));
+  orderedFill(nt, nv, tab, W, vOff, scanSh, [&](uint32_t i) { return uint32_t(s.iv[i]); },
+              [&](uint32_t i, uint32_t pos) { s.list[pos] = i; });
+}
+
 // Float sums that must follow the serial order (ascending track order inside
 // a vertex) are formed by a warp: the lanes evaluate 32 consecutive terms at
-// once and every lane adds them in order from the shuffles.  Terms of tracks
-// that the serial loop skips are +0.0, which leaves a sum unchanged (a sum
-// that starts at +0.0 never becomes -0.0 under round-to-nearest).
-
-// sum + the 32 lanes' terms, added in lane order (every lane gets the sum).
-// All 32 terms are added: the lanes past the vertex's tracks hold +0.0, which
-// leaves the sum unchanged.  Unrolled, the shuffles issue back to back and
-// only the additions form the dependent chain.
-__device__ __forceinline__ float laneOrderSum(float sum, float t) {
+// once, and K sums are formed together, lane k < K adding the 32 terms of the
+// k-th in order.  Terms of tracks that the serial loop skips are +0.0, which
+// leaves a sum unchanged (a sum that starts at +0.0 never becomes -0.0 under
+// round-to-nearest).  The terms go through shared memory, so that the K
+// chains of additions run side by side in K lanes: 40 instructions for all of
+// them, where shuffling each term to every lane took 64 for each sum.  Bound
+// by instruction issue on the event's one CTA.
+constexpr uint32_t kSumStride = 36;  // floats between the sums' terms: 16-byte rows in different banks
+constexpr uint32_t kSumWords = 4 * kSumStride;  // a warp's buffer
+template <int K>
+__device__ __forceinline__ void orderedSums(float* buf, const float (&term)[K], float& sum) {
+  const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
-  for (int l = 0; l < 32; ++l) sum += __shfl_sync(0xffffffffu, t, l);
-  return sum;
+  for (int k = 0; k < K; ++k) buf[k * kSumStride + lane] = term[k];
+  __syncwarp();
+  if (lane < K) {
+    const float4* row = reinterpret_cast<const float4*>(buf + lane * kSumStride);
+    float4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = row[j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      sum += v[j].x;
+      sum += v[j].y;
+      sum += v[j].z;
+      sum += v[j].w;
+    }
+  }
+  __syncwarp();
 }
 
 // fitVertices: weighted z, chi2 outlier rejection (iv = 9999), ndof and weight;
 // one warp per vertex
 __device__ void fitVertices(const VtxScratch& s, uint32_t nt, uint32_t nv, float chi2Max, float* zv, float* wv,
-                            float* chi2, int32_t* ndof, uint32_t* vOff, uint32_t* vCur, uint32_t* scanSh) {
-  groupByVertex(s, nt, nv, vOff, vCur, scanSh);
+                            float* chi2, int32_t* ndof, uint32_t* vOff, uint32_t* scanSh, float* sumBuf, uint16_t* tab,
+                            uint32_t tabBytes) {
+  groupByVertex(s, nt, nv, vOff, scanSh, tab, tabBytes);
   const uint32_t lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (uint32_t v = threadIdx.x >> 5; v < nv; v += nw) {
     const uint32_t b = vOff[v], n = vOff[v + 1] - b;
-    float z = 0, w = 0;
+    float zw = 0;  // lane 0: the sum of z, lane 1: of the weights
     for (uint32_t k0 = 0; k0 < n; k0 += 32) {
       const uint32_t k = k0 + lane;
-      float tz = 0.f, tw = 0.f;
+      float t[2] = {0.f, 0.f};
       if (k < n) {
         const uint32_t i = s.list[b + k];
         const float wi = 1.f / s.ezt2[i];
-        tz = s.zt[i] * wi;
-        tw = wi;
+        t[0] = s.zt[i] * wi;
+        t[1] = wi;
       }
-      z = laneOrderSum(z, tz);
-      w = laneOrderSum(w, tw);
+      orderedSums(sumBuf, t, zw);
     }
+    float z = __shfl_sync(0xffffffffu, zw, 0), w = __shfl_sync(0xffffffffu, zw, 1);
     z /= w;
     int32_t nd = -1;
     float c2s = 0;
     for (uint32_t k0 = 0; k0 < n; k0 += 32) {
       const uint32_t k = k0 + lane;
-      float t = 0.f;
+      float t[1] = {0.f};
       bool acc = false;
       if (k < n) {
         const uint32_t i = s.list[b + k];
@@ -210,12 +234,13 @@ __device__ void fitVertices(const VtxScratch& s, uint32_t nt, uint32_t nv, float
           s.iv[i] = 9999;
         } else {
           acc = true;
-          t = c2;
+          t[0] = c2;
         }
       }
       nd += __popc(__ballot_sync(0xffffffffu, acc));
-      c2s = laneOrderSum(c2s, t);
+      orderedSums(sumBuf, t, c2s);
     }
+    c2s = __shfl_sync(0xffffffffu, c2s, 0);
     if (nd > 0) w *= float(nd) / c2s;
     if (lane == 0) {
       zv[v] = z;
@@ -227,27 +252,101 @@ __device__ void fitVertices(const VtxScratch& s, uint32_t nt, uint32_t nv, float
   __syncthreads();
 }
 
+// lanes that share a track in the neighbour searches, and reductions over
+// them (called by whole warps)
+constexpr uint32_t kNbrLanes = 8;
+template <typename T, typename Op>
+__device__ __forceinline__ T groupReduce(T v, Op&& op) {
+#pragma unroll
+  for (uint32_t o = 1; o < kNbrLanes; o <<= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ uint32_t groupSum(uint32_t v) {
+  return groupReduce(v, [](uint32_t a, uint32_t b) { return a + b; });
+}
+__device__ __forceinline__ int32_t groupMax(int32_t v) {
+  return groupReduce(v, [](int32_t a, int32_t b) { return max(a, b); });
+}
+__device__ __forceinline__ int32_t groupMin(int32_t v) {
+  return groupReduce(v, [](int32_t a, int32_t b) { return min(a, b); });
+}
+__device__ __forceinline__ unsigned long long groupMin(unsigned long long v) {
+  return groupReduce(v, [](unsigned long long a, unsigned long long b) { return b < a ? b : a; });
+}
+
 // order-preserving map of a float to unsigned (negative values reversed)
 __device__ __forceinline__ uint32_t orderedBits(float x) {
   const uint32_t u = __float_as_uint(x);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// DBSCAN (gpuClusterTracksDBSCAN.h:16-227) and iterative
-// (gpuClusterTracksIterative.h:16-201) clustering after the neighbour counts:
+// The bins a track's candidates lie in: its own and the two next to it.
+__device__ __forceinline__ void candidateRange(const VtxScratch& s, const uint32_t* hoff, uint32_t i, uint32_t& pb,
+                                               uint32_t& pe) {
+  const int b0 = max(0, int(s.izt[i]) - 1), b1 = min(255, int(s.izt[i]) + 1);
+  pb = hoff[b0];
+  pe = hoff[b1 + 1];
+}
+
+// DBSCAN (gpuClusterTracksDBSCAN.h:16-227), first step, divided among the
+// CTAs as the neighbour counts are: every core track is linked (iv) to its
+// core neighbour of lowest z below its own, first in bin order among equal z;
+// a track whose candidates include a NaN is done by its first lane literally.
+__device__ void linkCores(const VtxScratch& s, uint32_t nt, const uint32_t* hoff, float eps, int32_t minT,
+                          uint32_t gFirst, uint32_t gStride, int32_t* iv) {
+  const uint32_t sub = threadIdx.x / kNbrLanes % (32 / kNbrLanes), gl = threadIdx.x % kNbrLanes;
+  const float* zP = s.zz;
+  const int32_t* nP = s.root;
+  for (uint32_t p0 = gFirst; p0 < nt; p0 += gStride) {
+    const uint32_t pi = p0 + sub;
+    const bool core = pi < nt && nP[pi] >= minT;
+    uint32_t pb = 0, pe = 0, i = 0, bestPos = 0xffffffffu;
+    float zi = 0.f;
+    if (core) {
+      i = s.hbins[pi];
+      candidateRange(s, hoff, i, pb, pe);
+      zi = zP[pi];
+    }
+    float bestZ = zi;
+    int32_t nan = isnan(zi) ? 1 : 0;
+    for (uint32_t p = pb + gl; p < pe; p += kNbrLanes) {
+      const float zj = zP[p];
+      if (isnan(zj)) nan = 1;
+      if (zj < bestZ && nP[p] >= minT && !(fabsf(zi - zj) > eps)) {
+        bestZ = zj;
+        bestPos = p;
+      }
+    }
+    nan = groupMax(nan);
+    const unsigned long long best = groupMin(
+        bestPos == 0xffffffffu ? ~0ull : (uint64_t(orderedBits(bestZ)) << 32) | bestPos);
+    if (nan) {
+      if (gl == 0) {  // the serial loop as written
+        float mz = zi;
+        for (uint32_t p = pb; p < pe; ++p) {
+          if (zP[p] >= mz || nP[p] < minT || fabsf(zi - zP[p]) > eps) continue;
+          mz = zP[p];
+          iv[i] = int32_t(s.hbins[p]);
+        }
+      }
+    } else if (gl == 0 && best != ~0ull) {
+      iv[i] = int32_t(s.hbins[uint32_t(best & 0xffffffffu)]);
+    }
+  }
+}
+
+// The rest of DBSCAN and the iterative clustering
+// (gpuClusterTracksIterative.h:16-201) after the neighbour counts:
 // iv[i] left pointing at track i's root (the numbering that follows is the
-// one of the density clusterer).  One block; warp per track for the
+// one of the density clusterer).  One block; kNbrLanes lanes per track for the
 // neighbour loops, whose serial order is reproduced by (key, position)
-// reductions; a track whose candidates include a NaN is done by lane 0
+// reductions; a track whose candidates include a NaN is done by its first lane
 // literally.
 __device__ void clusterCoresAndEdges(const VtxScratch& s, uint32_t nt, const uint32_t* hoff, int algo, float eps,
                                      float chi2max, int32_t minT, int* sFlag) {
-  const uint32_t lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  auto range = [&](uint32_t i, uint32_t& pb, uint32_t& pe) {
-    const int b0 = max(0, int(s.izt[i]) - 1), b1 = min(255, int(s.izt[i]) + 1);
-    pb = hoff[b0];
-    pe = hoff[b1 + 1];
-  };
+  const uint32_t sub = threadIdx.x / kNbrLanes % (32 / kNbrLanes), gl = threadIdx.x % kNbrLanes;
+  const uint32_t gFirst = threadIdx.x / 32 * (32 / kNbrLanes), gStride = blockDim.x / kNbrLanes;
+  auto range = [&](uint32_t i, uint32_t& pb, uint32_t& pe) { candidateRange(s, hoff, i, pb, pe); };
   auto percolate = [&]() {
     for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
       int32_t m = s.iv[i];
@@ -258,44 +357,12 @@ __device__ void clusterCoresAndEdges(const VtxScratch& s, uint32_t nt, const uin
     for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) s.iv[i] = s.root[i];
     __syncthreads();
   };
+  // z, its error and the neighbour count in histogram order; the counts' place
+  // (root) is free for the percolation once the cores are linked
+  const float* zP = s.zz;
+  const float* eP = reinterpret_cast<const float*>(s.list);
+  const int32_t* nP = s.root;
   if (algo == 1) {
-    // core tracks: the core neighbour of lowest z below the track's own
-    // (first in bin order among equal z)
-    for (uint32_t i = threadIdx.x >> 5; i < nt; i += nw) {
-      if (s.nn[i] < minT) continue;
-      uint32_t pb, pe;
-      range(i, pb, pe);
-      const float zi = s.zt[i];
-      unsigned long long best = ~0ull;
-      bool nan = isnan(zi);
-      for (uint32_t p = pb + lane; p < pe; p += 32) {
-        const uint32_t j = s.hbins[p];
-        const float zj = s.zt[j];
-        nan |= isnan(zj);
-        if (!(zj < zi) || s.nn[j] < minT || fabsf(zi - zj) > eps) continue;
-        const unsigned long long key = (uint64_t(orderedBits(zj)) << 32) | p;
-        best = key < best ? key : best;
-      }
-      if (__any_sync(0xffffffffu, nan)) {
-        if (lane == 0) {  // the serial loop as written
-          float mz = zi;
-          for (uint32_t p = pb; p < pe; ++p) {
-            const uint32_t j = s.hbins[p];
-            if (s.zt[j] >= mz || s.nn[j] < minT || fabsf(zi - s.zt[j]) > eps) continue;
-            mz = s.zt[j];
-            s.iv[i] = int32_t(j);
-          }
-        }
-        continue;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-        best = other < best ? other : best;
-      }
-      if (lane == 0 && best != ~0ull) s.iv[i] = int32_t(s.hbins[uint32_t(best & 0xffffffffu)]);
-    }
-    __syncthreads();
     percolate();
   } else {
     // connected components of the compatible core tracks: every label
@@ -304,21 +371,26 @@ __device__ void clusterCoresAndEdges(const VtxScratch& s, uint32_t nt, const uin
     for (uint32_t it = 0; it <= nt + 1; ++it) {
       if (threadIdx.x == 0) *sFlag = 0;
       __syncthreads();
-      for (uint32_t i = threadIdx.x >> 5; i < nt; i += nw) {
-        if (s.nn[i] < minT) continue;
-        uint32_t pb, pe;
-        range(i, pb, pe);
-        const float zi = s.zt[i], ei = s.ezt2[i];
-        int32_t m = s.iv[i];
-        for (uint32_t p = pb + lane; p < pe; p += 32) {
-          const uint32_t j = s.hbins[p];
-          if (j == i || s.nn[j] < minT) continue;
-          const float dist = fabsf(zi - s.zt[j]);
-          if (dist > eps || dist * dist > chi2max * (ei + s.ezt2[j])) continue;
-          m = min(m, s.iv[j]);
+      for (uint32_t p0 = gFirst; p0 < nt; p0 += gStride) {
+        const uint32_t pi = p0 + sub, i = pi < nt ? s.hbins[pi] : 0u;
+        const bool core = pi < nt && nP[pi] >= minT;
+        uint32_t pb = 0, pe = 0;
+        float zi = 0.f, ei = 0.f;
+        int32_t m = 0;
+        if (core) {
+          range(i, pb, pe);
+          zi = zP[pi];
+          ei = eP[pi];
+          m = s.iv[i];
         }
-        m = __reduce_min_sync(0xffffffffu, m);
-        if (lane == 0 && m < s.iv[i]) {
+        for (uint32_t p = pb + gl; p < pe; p += kNbrLanes) {
+          if (p == pi || nP[p] < minT) continue;
+          const float dist = fabsf(zi - zP[p]);
+          if (dist > eps || dist * dist > chi2max * (ei + eP[p])) continue;
+          m = min(m, s.iv[s.hbins[p]]);
+        }
+        m = groupMin(m);
+        if (gl == 0 && core && m < s.iv[i]) {
           atomicMin(&s.iv[i], m);
           *sFlag = 1;
         }
@@ -339,43 +411,43 @@ __device__ void clusterCoresAndEdges(const VtxScratch& s, uint32_t nt, const uin
   }
   // edge rule: a non-core track joins its closest chi2-compatible core
   // neighbour (last in bin order among equal distances)
-  for (uint32_t i = threadIdx.x >> 5; i < nt; i += nw) {
-    if (s.nn[i] >= minT) continue;
-    uint32_t pb, pe;
-    range(i, pb, pe);
-    const float zi = s.zt[i], ei = s.ezt2[i];
+  for (uint32_t p0 = gFirst; p0 < nt; p0 += gStride) {
+    const uint32_t pi = p0 + sub, i = pi < nt ? s.hbins[pi] : 0u;
+    const bool edge = pi < nt && s.nn[i] < minT;
+    uint32_t pb = 0, pe = 0;
+    float zi = 0.f, ei = 0.f;
+    if (edge) {
+      range(i, pb, pe);
+      zi = zP[pi];
+      ei = eP[pi];
+    }
     unsigned long long best = ~0ull;
-    bool nan = false;
-    for (uint32_t p = pb + lane; p < pe; p += 32) {
-      const uint32_t j = s.hbins[p];
-      if (s.nn[j] < minT) continue;
-      const float dist = fabsf(zi - s.zt[j]);
-      nan |= isnan(dist) || isnan(chi2max * (ei + s.ezt2[j]));
-      if (dist > eps || dist * dist > chi2max * (ei + s.ezt2[j])) continue;
+    int32_t nan = 0;
+    for (uint32_t p = pb + gl; p < pe; p += kNbrLanes) {
+      if (s.nn[s.hbins[p]] < minT) continue;
+      const float dist = fabsf(zi - zP[p]), reach = chi2max * (ei + eP[p]);
+      if (isnan(dist) || isnan(reach)) nan = 1;
+      if (dist > eps || dist * dist > reach) continue;
       const unsigned long long key = (uint64_t(__float_as_uint(dist)) << 32) | uint64_t(0xffffffffu - p);
       best = key < best ? key : best;
     }
-    if (__any_sync(0xffffffffu, nan)) {
-      if (lane == 0) {
-        s.root[i] = s.iv[i];
-        float mdist = eps;
-        for (uint32_t p = pb; p < pe; ++p) {
-          const uint32_t j = s.hbins[p];
-          if (s.nn[j] < minT) continue;
-          const float dist = fabsf(zi - s.zt[j]);
-          if (dist > mdist || dist * dist > chi2max * (ei + s.ezt2[j])) continue;
-          mdist = dist;
-          s.root[i] = s.iv[j];
-        }
+    nan = groupMax(nan);
+    best = groupMin(best);
+    if (!edge || gl != 0) continue;  // (no reduction follows in this step)
+    if (nan) {
+      s.root[i] = s.iv[i];
+      float mdist = eps;
+      for (uint32_t p = pb; p < pe; ++p) {
+        const uint32_t j = s.hbins[p];
+        if (s.nn[j] < minT) continue;
+        const float dist = fabsf(zi - s.zt[j]);
+        if (dist > mdist || dist * dist > chi2max * (ei + s.ezt2[j])) continue;
+        mdist = dist;
+        s.root[i] = s.iv[j];
       }
       continue;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-      best = other < best ? other : best;
-    }
-    if (lane == 0) s.root[i] = best != ~0ull ? s.iv[s.hbins[0xffffffffu - uint32_t(best & 0xffffffffu)]] : s.iv[i];
+    s.root[i] = best != ~0ull ? s.iv[s.hbins[0xffffffffu - uint32_t(best & 0xffffffffu)]] : s.iv[i];
   }
   __syncthreads();
   // edge tracks take their core's root; the others keep theirs
@@ -384,7 +456,7 @@ __device__ void clusterCoresAndEdges(const VtxScratch& s, uint32_t nt, const uin
   __syncthreads();
 }
 
-// Launched as a cluster of P CTAs per event (P = 1 for large batches).  With
+// Launched as a cluster of P CTAs per event (pairs for large batches).  With
 // P > 1 and the per-track arrays in shared memory, every CTA builds the track
 // arrays and the z histogram, the two neighbour searches are divided among the
 // CTAs by track, each result written into every CTA's shared memory, and rank
@@ -439,15 +511,16 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
   // CTAs' counts place every run, and a second walk writes the selected tracks
   // in ascending order (into every CTA's shared memory, or the global
   // scratch).  The selection of each step is kept as a bit when the range has
-  // at most 32 steps, else evaluated again.
+  // at most 64 steps, else evaluated again.
   const uint32_t g0 = uint32_t(uint64_t(guard) * rank / P), g1 = uint32_t(uint64_t(guard) * (rank + 1) / P);
   for (uint32_t t = g0 + threadIdx.x; t < g1; t += blockDim.x) idv[t] = -1;
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t R = (g1 - g0 + nw * 32 - 1) / (nw * 32) * 32;
   const uint32_t w0 = min(g1, g0 + warp * R), w1 = min(g1, w0 + R);
   const uint32_t steps = (w1 - w0 + 31) / 32;
-  const bool keepBits = steps <= 32;
-  uint32_t cnt = 0, bits = 0;
+  const bool keepBits = steps <= 64;
+  uint32_t cnt = 0;
+  uint64_t bits = 0;
   for (uint32_t k = 0; k < steps; k += 4) {
     bool sel[4];
 #pragma unroll
@@ -457,7 +530,7 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
     }
 #pragma unroll
     for (uint32_t u = 0; u < 4; ++u) {
-      if (sel[u] && keepBits) bits |= 1u << (k + u);
+      if (sel[u] && keepBits) bits |= uint64_t(1) << (k + u);
       cnt += __popc(__ballot_sync(0xffffffffu, sel[u]));
     }
   }
@@ -481,15 +554,18 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
   __syncthreads();
   // The count decides where the per-track arrays live: in the shared memory
   // of every CTA, or once in the global scratch.  The neighbour searches are
-  // split among the cluster's CTAs (the density clusterer); their results go
+  // split among the cluster's CTAs (not the iterative clusterer's); their results go
   // to every CTA's shared memory, or once to the global scratch.
   const bool smemPath = sNt <= kSmemTracks;
   const VtxScratch s = smemPath ? carve(vsm, kSmemTracks) : scratchOf(ws, e);
-  const bool split = P > 1 && algo == 0;
+  const bool split = P > 1 && algo != 2;
   const bool remote = split && smemPath;       // results written into every CTA
   const bool active = split || rank == 0;      // CTAs that take part in the searches
   const bool writer = smemPath || rank == 0;   // CTAs that build their own track arrays
-  const uint32_t wFirst = split ? rank * nw : 0, wStride = split ? P * nw : nw;
+  // the searches' tracks: kNbrLanes lanes each, 32 / kNbrLanes tracks per warp
+  const uint32_t sub = lane / kNbrLanes, gl = lane % kNbrLanes;
+  const uint32_t gFirst = ((split ? rank * nw : 0u) + (threadIdx.x >> 5)) * (32 / kNbrLanes);
+  const uint32_t gStride = (split ? P * nw : nw) * (32 / kNbrLanes);
   // every CTA places its selected tracks; in the shared-memory path each
   // track goes to every CTA that works on it (all with the split, else rank 0)
   const uint32_t nDst = smemPath ? (split ? P : 1u) : 1u;
@@ -530,12 +606,9 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
 
   if (active) {
   // ---- clusterTracksByDensity: z histogram (256 bins of 1 mm)
-  for (uint32_t b = threadIdx.x; b < 257; b += blockDim.x) hoff[b] = 0;
-  __syncthreads();
   for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
     int iz = int(double(s.zt[i]) * 10.);
     iz = min(max(iz, -128), 127);
-    atomicAdd(&hoff[iz + 128], 1u);
     if (writer) {
       s.izt[i] = uint8_t(iz + 128);
       s.iv[i] = int32_t(i);
@@ -543,45 +616,18 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
     }
   }
   __syncthreads();
-  {
-    uint32_t carry = 0;
-    for (uint32_t b0 = 0; b0 < 257; b0 += blockDim.x) {
-      uint32_t b = b0 + threadIdx.x;
-      uint32_t v = b < 257 ? hoff[b] : 0u;
-      uint32_t tot;
-      uint32_t pre = blockExclusiveScan(v, scanSh, &tot);
-      if (b < 257) hoff[b] = carry + pre;
-      carry += tot;
-    }
-  }
-  __syncthreads();
-  // the serial fill stores each bin in descending track order.  Warp w owns
-  // bins [8 w, 8 w + 8) and walks the tracks once from the last one down,
-  // 32 at a time: lanes holding the same bin are ranked among themselves
-  // (match), and the bin's cursor advances by their number.
+  // The serial fill stores each bin in descending track order: the items are
+  // the tracks from the last one down.  In the global-scratch path every CTA
+  // needs the bins' starts, and rank 0 writes their content; a CTA cannot
+  // read another's izt before the cluster barrier, so each forms its own.
+  static_assert(kVtxThreads / 32 * 256 * 2 <= kSmemTracks * 4, "the histogram's table in root");
+  orderedFill(nt, 256, smemPath ? reinterpret_cast<uint16_t*>(s.root) : reinterpret_cast<uint16_t*>(vsm), nw, hoff,
+              scanSh,
+              [&](uint32_t r) { return uint32_t(min(max(int(double(s.zt[nt - 1 - r]) * 10.), -128), 127) + 128); },
+              [&](uint32_t r, uint32_t pos) {
+                if (writer) s.hbins[pos] = uint16_t(nt - 1 - r);
+              });
   if (writer) {
-    uint32_t* cur = vCur;  // free until the vertex fit: per-bin fill cursors
-    for (uint32_t b = threadIdx.x; b < 256; b += blockDim.x) cur[b] = hoff[b];
-    __syncthreads();
-    const uint32_t bpw = (256 + nw - 1) / nw, bLo = (threadIdx.x >> 5) * bpw, bHi = min(256u, bLo + bpw);
-    for (uint32_t r0 = 0; r0 < nt && bLo < bHi; r0 += 32) {
-      const uint32_t r = r0 + lane;
-      const uint32_t i = nt - 1 - r;
-      const uint32_t b = r < nt ? s.izt[i] : 0xffffu;
-      const bool in = b >= bLo && b < bHi;
-      const uint32_t m = __ballot_sync(0xffffffffu, in);
-      if (m) {
-        const uint32_t peers = __match_any_sync(0xffffffffu, in ? b : 0xffffffffu) & m;
-        if (in) {
-          const uint32_t pos = cur[b] + __popc(peers & lanemaskLt());
-          s.hbins[pos] = uint16_t(i);
-          __syncwarp(peers);
-          if ((peers & lanemaskLt()) == 0) cur[b] += __popc(peers);
-        }
-        __syncwarp();
-      }
-    }
-    __syncthreads();
     // z and its error of every track in histogram order, so that the
     // neighbour searches read their candidates contiguously (zz and list are
     // free until the fits)
@@ -603,84 +649,115 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
   const float* eP = reinterpret_cast<const float*>(s.list);
   int32_t* nP = s.root;  // free until the percolation
   if (active) {
-  // neighbour counts: one warp per track (taken in histogram order), the
-  // lanes take 32 consecutive entries of the track's three bins at a time.
-  // Each count is kept by track (nn) and by histogram position (nP).
-  for (uint32_t pi = wFirst + (threadIdx.x >> 5); pi < nt; pi += wStride) {
-    const uint32_t i = s.hbins[pi];
-    const float zi = zP[pi], ei = eP[pi];
-    uint32_t cnt = 0;  // per lane, summed once per track
-    if (!(ei > er2mx)) {
-      const int b0 = max(0, int(s.izt[i]) - 1), b1 = min(255, int(s.izt[i]) + 1);
-      const uint32_t pb = hoff[b0], pe = hoff[b1 + 1];
-      for (uint32_t p = pb + lane; p < pe; p += 32) {
-        const uint32_t j = s.hbins[p];
-        const float dist = fabsf(zi - zP[p]);
-        cnt += (i != j && !(dist > eps) && (algo == 1 || !(dist * dist > chi2max * (ei + eP[p])))) ? 1u : 0u;
+  // neighbour counts: kNbrLanes lanes per track (taken in histogram order)
+  // share the entries of the track's three bins.  Each count is kept by track
+  // (nn) and by histogram position (nP).  A track has a few tens of
+  // candidates: a warp per track left most of its instructions in the
+  // reductions (1087 tracks: 8k and, for the closest denser neighbour below,
+  // 17k of the kernel's 113k cycles).
+  for (uint32_t p0 = gFirst; p0 < nt; p0 += gStride) {
+    const uint32_t pi = p0 + sub;
+    uint32_t cnt = 0, i = 0;
+    if (pi < nt) {
+      i = s.hbins[pi];
+      const float zi = zP[pi], ei = eP[pi];
+      if (!(ei > er2mx)) {
+        const int b0 = max(0, int(s.izt[i]) - 1), b1 = min(255, int(s.izt[i]) + 1);
+        const uint32_t pb = hoff[b0], pe = hoff[b1 + 1];
+        for (uint32_t p = pb + gl; p < pe; p += kNbrLanes) {
+          const float dist = fabsf(zi - zP[p]);
+          // a track is not its own neighbour: its histogram position is pi
+          cnt += (p != pi && !(dist > eps) && (algo == 1 || !(dist * dist > chi2max * (ei + eP[p])))) ? 1u : 0u;
+        }
       }
-      cnt = __reduce_add_sync(0xffffffffu, cnt);
     }
-    if (remote ? lane < P : lane == 0) {
-      *(remote ? cl.map_shared_rank(s.nn, lane) + i : s.nn + i) = int32_t(cnt);
-      *(remote ? cl.map_shared_rank(nP, lane) + pi : nP + pi) = int32_t(cnt);
+    cnt = groupSum(cnt);
+    if (pi < nt) {
+      if (remote) {
+        for (uint32_t r = gl; r < P; r += kNbrLanes) {
+          cl.map_shared_rank(s.nn, r)[i] = int32_t(cnt);
+          cl.map_shared_rank(nP, r)[pi] = int32_t(cnt);
+        }
+      } else if (gl == 0) {
+        s.nn[i] = int32_t(cnt);
+        nP[pi] = int32_t(cnt);
+      }
     }
   }
   }
   // every CTA holds every neighbour count
   cl.sync();
-  if (active && algo != 0) clusterCoresAndEdges(s, nt, hoff, algo, eps, chi2max, 2, &sFlag);
+  // only rank 0 goes on after the searches: their results go there
+  int32_t* const ivOut = remote ? cl.map_shared_rank(s.iv, 0) : s.iv;
+  if (active && algo == 1) linkCores(s, nt, hoff, eps, 2, gFirst, gStride, ivOut);
   if (active && algo == 0) {
   // Closest denser neighbour.  The serial loop (mdist starts at eps; a
   // candidate is taken when denser, not farther than mdist and
   // chi2-compatible) ends on the last candidate of minimal distance among the
-  // qualifying ones -- unless a candidate with a NaN distance qualifies: from
-  // then on every denser, chi2-compatible candidate is taken, so the result
-  // is the last of those.  The warp evaluates both, the first as the minimum
-  // of (distance, reversed position).
-  for (uint32_t pi = wFirst + (threadIdx.x >> 5); pi < nt; pi += wStride) {
-    const uint32_t i = s.hbins[pi];
-    const int b0 = max(0, int(s.izt[i]) - 1), b1 = min(255, int(s.izt[i]) + 1);
-    const uint32_t pb = hoff[b0], pe = hoff[b1 + 1];
-    const float zi = zP[pi], ei = eP[pi];
-    const int32_t ni = nP[pi];
-    // per-lane running results, combined once per track
-    unsigned long long bestKey = ~0ull;
-    bool nanLane = false;
-    int32_t lastOk = -1;
-    for (uint32_t p = pb + lane; p < pe; p += 32) {
+  // qualifying ones: each lane runs it over its candidates, and the lanes'
+  // results are combined as the minimum of (distance, reversed position).  A
+  // track with a denser candidate at a NaN distance runs the serial loop.
+  for (uint32_t p0 = gFirst; p0 < nt; p0 += gStride) {
+    const uint32_t pi = p0 + sub;
+    uint32_t i = 0;
+    // per lane, in ascending position: the closest so far (the last of equal
+    // distances) and whether a NaN distance was met
+    float bestDist = eps;
+    uint32_t bestPos = 0xffffffffu;
+    int32_t nan = 0;
+    uint32_t pb = 0, pe = 0;
+    float zi = 0.f, ei = 0.f;
+    int32_t ni = 0;
+    auto denser = [&](uint32_t p) {
       const int32_t nj = nP[p];
-      const float zj = zP[p];
-      const float dist = fabsf(zi - zj);
-      const bool dens = !(nj < ni) && !(nj == ni && zj >= zi);
-      const bool dc = dens && !(dist * dist > chi2max * (ei + eP[p]));
-      nanLane |= dens && isnan(dist);
-      if (dc) {
-        lastOk = int32_t(p);
-        if (!(dist > eps)) {
-          const unsigned long long key = (uint64_t(__float_as_uint(dist)) << 32) | uint64_t(0xffffffffu - p);
-          bestKey = key < bestKey ? key : bestKey;
+      return !(nj < ni) && !(nj == ni && zP[p] >= zi);
+    };
+    auto near = [&](float dist, uint32_t p) { return !(dist * dist > chi2max * (ei + eP[p])); };
+    if (pi < nt) {
+      i = s.hbins[pi];
+      const int b0 = max(0, int(s.izt[i]) - 1), b1 = min(255, int(s.izt[i]) + 1);
+      pb = hoff[b0];
+      pe = hoff[b1 + 1];
+      zi = zP[pi];
+      ei = eP[pi];
+      ni = nP[pi];
+      for (uint32_t p = pb + gl; p < pe; p += kNbrLanes) {
+        const float dist = fabsf(zi - zP[p]);
+        if (!denser(p)) continue;
+        if (isnan(dist)) nan = 1;
+        if (dist <= bestDist && near(dist, p)) {
+          bestDist = dist;
+          bestPos = p;
         }
       }
     }
-    const bool anyNaN = __any_sync(0xffffffffu, nanLane);
-    lastOk = __reduce_max_sync(0xffffffffu, lastOk);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xffffffffu, bestKey, o);
-      bestKey = other < bestKey ? other : bestKey;
-    }
+    nan = groupMax(nan);
+    const unsigned long long bestKey =
+        groupMin(bestPos == 0xffffffffu
+                     ? ~0ull
+                     : (uint64_t(__float_as_uint(bestDist)) << 32) | uint64_t(0xffffffffu - bestPos));
     int32_t best = int32_t(i);
-    if (anyNaN)
-      best = int32_t(s.hbins[lastOk]);
-    else if (bestKey != ~0ull)
-      best = int32_t(s.hbins[0xffffffffu - uint32_t(bestKey & 0xffffffffu)]);
-    if (remote ? lane < P : lane == 0) *(remote ? cl.map_shared_rank(s.iv, lane) + i : s.iv + i) = best;
+    if (pi < nt) {
+      if (nan) {
+        // the serial loop as written
+        float mdist = eps;
+        for (uint32_t p = pb; p < pe; ++p) {
+          const float dist = fabsf(zi - zP[p]);
+          if (!denser(p) || dist > mdist || !near(dist, p)) continue;
+          mdist = dist;
+          best = int32_t(s.hbins[p]);
+        }
+      } else if (bestKey != ~0ull)
+        best = int32_t(s.hbins[0xffffffffu - uint32_t(bestKey & 0xffffffffu)]);
+      if (gl == 0) ivOut[i] = best;
+    }
   }
   }
-  // every CTA holds every closest denser neighbour; only rank 0 goes on,
-  // and no CTA reads another CTA's shared memory after this point
+  // rank 0 holds every track's link and goes on alone; no CTA reads another
+  // CTA's shared memory after this point
   cl.sync();
   if (rank != 0) return;
+  if (algo != 0) clusterCoresAndEdges(s, nt, hoff, algo, eps, chi2max, 2, &sFlag);
   // percolate to the seed
   for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
     int32_t m = s.iv[i];
@@ -719,8 +796,18 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
     found = kMaxVtx - 1;
   }
 
+  // the grouping's table and the warps' sum buffers (used in turn): the place of
+  // nn and root, free from here on, or the dynamic shared memory that the
+  // global-scratch path leaves unused
+  static_assert(kVtxThreads / 32 * kSumWords <= kSmemTracks && 5 * kSmemTracks % 4 == 0, "sum buffers in nn, aligned");
+  static_assert(2 * kSmemTracks * 4 / 2 / kMaxVtx >= 1, "a table row for every vertex in nn and root");
+  char* const spare = smemPath ? reinterpret_cast<char*>(s.nn) : vsm;
+  float* const sumBuf = reinterpret_cast<float*>(spare) + (threadIdx.x >> 5) * kSumWords;
+  uint16_t* const tab = reinterpret_cast<uint16_t*>(spare);
+  const uint32_t tabBytes = smemPath ? 2 * kSmemTracks * 4 : uint32_t(kVtxSmemBytes);
+
   // ---- fitVertices(50)
-  fitVertices(s, nt, found, 50.f, zv, wv, vchi2, ndof, vOff, vCur, scanSh);
+  fitVertices(s, nt, found, 50.f, zv, wv, vchi2, ndof, vOff, scanSh, sumBuf, tab, tabBytes);
 
   // ---- splitVertices(9): tracks of each vertex are the list built by the fit
   //      minus the ones rejected there (iv = 9999)
@@ -747,30 +834,28 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
     bool more = true;
     while (more) {
       more = false;
-      znew[0] = znew[1] = 0;
-      wnew[0] = wnew[1] = 0;
+      float sums = 0;  // lanes 0..3: z and weight of the first half, of the second
       for (uint32_t k0 = 0; k0 < n; k0 += 32) {
         const uint32_t k = k0 + lane;
-        float z0 = 0.f, w0 = 0.f, z1 = 0.f, w1 = 0.f;
+        float t[4] = {0.f, 0.f, 0.f, 0.f};
         if (k < n) {
           const uint32_t i = s.list[b + k];
           if (s.iv[i] == int32_t(kv)) {
             const float ww = 1.f / s.ezt2[i];
             const float p = s.zz[i] * ww;
-            if (s.newV[i]) {
-              z1 = p;
-              w1 = ww;
-            } else {
-              z0 = p;
-              w0 = ww;
-            }
+            const bool second = s.newV[i] != 0;
+            t[0] = second ? 0.f : p;
+            t[1] = second ? 0.f : ww;
+            t[2] = second ? p : 0.f;
+            t[3] = second ? ww : 0.f;
           }
         }
-        znew[0] = laneOrderSum(znew[0], z0);
-        wnew[0] = laneOrderSum(wnew[0], w0);
-        znew[1] = laneOrderSum(znew[1], z1);
-        wnew[1] = laneOrderSum(wnew[1], w1);
+        orderedSums(sumBuf, t, sums);
       }
+      znew[0] = __shfl_sync(0xffffffffu, sums, 0);
+      wnew[0] = __shfl_sync(0xffffffffu, sums, 1);
+      znew[1] = __shfl_sync(0xffffffffu, sums, 2);
+      wnew[1] = __shfl_sync(0xffffffffu, sums, 3);
       znew[0] /= wnew[0];
       znew[1] /= wnew[1];
       bool changed = false;
@@ -827,7 +912,7 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
   }
 
   // ---- fitVertices(5000)
-  fitVertices(s, nt, nv, 5000.f, zv, wv, vchi2, ndof, vOff, vCur, scanSh);
+  fitVertices(s, nt, nv, 5000.f, zv, wv, vchi2, ndof, vOff, scanSh, sumBuf, tab, tabBytes);
 
   // ---- sortByPt2
   if (threadIdx.x == 0) c->nVertices = nv;
@@ -839,12 +924,12 @@ __global__ void __launch_bounds__(kVtxThreads) kVertices(Workspace ws, int algo)
     float p2 = 0;
     for (uint32_t k0 = 0; k0 < n; k0 += 32) {
       const uint32_t k = k0 + lane;
-      float t = 0.f;
+      float t[1] = {0.f};
       if (k < n) {
         const uint32_t i = s.list[b + k];
-        if (s.iv[i] <= 9990) t = s.ptt2[i];
+        if (s.iv[i] <= 9990) t[0] = s.ptt2[i];
       }
-      p2 = laneOrderSum(p2, t);
+      orderedSums(sumBuf, t, p2);
     }
     if (lane == 0) ptv2[v] = p2;
   }
@@ -878,12 +963,14 @@ cudaError_t runVertices(Workspace& ws, uint32_t nEvents, cudaStream_t stream, in
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }
-  // small batches: a cluster of kVtxCtas CTAs per event shortens the event's
-  // latency; large batches: pairs of CTAs (measured at 64 PU50 events: 0.52 ->
-  // 0.39 ms per batch and +2 % throughput with three batches in flight).  Only
-  // the density clusterer splits its work across the cluster; the others run
-  // on one CTA.
-  const uint32_t P = algo != 0 ? 1u : (nEvents <= kClusterMaxEvents ? kVtxCtas : 2u);
+  // small batches: a cluster of kVtxCtas CTAs per event, as many as the SMs
+  // hold (a CTA's shared memory takes one whole), shortens the event's
+  // latency (8 instead of 4: 93k -> 52k cycles for walking the 318k tuples of a
+  // PU200 event); large batches: pairs of CTAs (measured at 64 PU50 events:
+  // 0.52 -> 0.39 ms per batch and +2 % throughput with three batches in
+  // flight).  The iterative clusterer does its searches on one CTA; there the
+  // others share the loading only.
+  const uint32_t P = nEvents <= kClusterMaxEvents ? kVtxCtas : (nEvents <= 2 * kClusterMaxEvents ? 4u : 2u);
   cudaError_t le = cudaSuccess;
   PG_PROBED("kVertices", stream,
             le = launchClustered(kVertices, P, nEvents, kVtxThreads, kVtxSmemBytes, stream, ws, algo));
