@@ -342,11 +342,9 @@ int captureGraph(pg_ctx* c, Slot& s, uint32_t n, cudaGraphExec_t* out) {
   if (pr) pr->used = 0;
   tProbe = pr;
   s.ws.tune = tuningFor(c, n);
-  cudaError_t le = runChain(c->des, s.ws, n, s.stream, c->cfg.riemann_fit != 0, int(c->cfg.vertex_algo));
-  if (le == cudaSuccess) {
-    launchPack(s.ws, n, s.dRes, s.stream);
-    le = cudaGetLastError();
-  }
+  cudaError_t le =
+      runChain(c->des, s.ws, n, s.stream, s.side, s.dRes, c->cfg.riemann_fit != 0, int(c->cfg.vertex_algo));
+  if (le == cudaSuccess) le = cudaGetLastError();
   tProbe = nullptr;
   s.probeUsed[n] = pr ? pr->used : 0;
   e = cudaStreamEndCapture(s.stream, &g);
@@ -397,8 +395,8 @@ int pixgpu::launchBatch(pg_ctx* c, Slot& s) {
     if (pr) pr->used = 0;
     tProbe = pr;
     s.ws.tune = tuningFor(c, s.nEvents);
-    e = runChain(c->des, s.ws, s.nEvents, s.stream, c->cfg.riemann_fit != 0, int(c->cfg.vertex_algo));
-    if (e == cudaSuccess) launchPack(s.ws, s.nEvents, s.dRes, s.stream);
+    e = runChain(c->des, s.ws, s.nEvents, s.stream, s.side, s.dRes, c->cfg.riemann_fit != 0,
+                 int(c->cfg.vertex_algo));
     tProbe = nullptr;
     s.lastProbeUsed = pr ? pr->used : 0;
     if (e != cudaSuccess) return cudaFail(c, e, "chain launch");
@@ -465,6 +463,9 @@ int createSlot(pg_ctx* c, Slot& s, size_t bytes) {
   s.ws.ca.lateFishbone = c->cfg.late_fishbone != 0;
   s.ws.ca.mixedFit = c->cfg.mixed_fit != 0;
   if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&s.side.stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&s.side.fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&s.side.join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&s.gathered, cudaEventDisableTiming) != cudaSuccess ||
       cudaMallocHost(&s.hWords, size_t(c->cfg.max_words_per_batch) * 4) != cudaSuccess ||
@@ -521,6 +522,7 @@ int createSlot(pg_ctx* c, Slot& s, size_t bytes) {
 
 void destroySlot(Slot& s) {
   if (s.stream) cudaStreamSynchronize(s.stream);
+  if (s.side.stream) cudaStreamSynchronize(s.side.stream);
   for (auto& g : s.graphs) cudaGraphExecDestroy(g.second);
   s.graphs.clear();
   if (s.probe) {
@@ -536,6 +538,9 @@ void destroySlot(Slot& s) {
   if (s.dRefs) cudaFree(s.dRefs);
   if (s.done) cudaEventDestroy(s.done);
   if (s.gathered) cudaEventDestroy(s.gathered);
+  if (s.side.fork) cudaEventDestroy(s.side.fork);
+  if (s.side.join) cudaEventDestroy(s.side.join);
+  if (s.side.stream) cudaStreamDestroy(s.side.stream);
   if (s.stream) cudaStreamDestroy(s.stream);
   if (s.hWords) cudaFreeHost(s.hWords);
   if (s.hFed) cudaFreeHost(s.hFed);

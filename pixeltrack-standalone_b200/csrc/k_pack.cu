@@ -1,6 +1,6 @@
 // Result packing and small batch-setup kernels.
 //
-// kPackResults writes, per event, the compact result that a consumer of the
+// kPackTracks writes, per event, the compact result that a consumer of the
 // chain needs (the role of the PixelTrackSoAFromCUDA / PixelVertexSoAFromCUDA
 // transfer modules of the CUDA program): counts, the loose tracks (quality >=
 // loose, in tuple order) with their fit state, covariance, hits and vertex
@@ -56,7 +56,10 @@ constexpr uint32_t kPackCtas = 8;  // CTAs per event in a small batch
 // dynamic shared memory: the slice's loose tuple indices and the whole list
 constexpr size_t kPackSmemBytes = 2 * size_t(kResultTracks) * sizeof(uint32_t);
 
-__global__ void __launch_bounds__(512) kPackResults(Workspace ws, uint8_t* out) {
+// The tracks, everything of them but their vertex: it needs nothing from the
+// vertex finder and runs beside it (runVerticesAndPack).  The loose tuples'
+// list stays in ws.candidates for kPackVertices.
+__global__ void __launch_bounds__(512) kPackTracks(Workspace ws, uint8_t* out) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const uint32_t r = cl.block_rank(), P = cl.num_blocks();
@@ -143,16 +146,34 @@ __global__ void __launch_bounds__(512) kPackResults(Workspace ws, uint8_t* out) 
     const uint32_t t = sIdx[i / 5], k = i % 5;
     w32[i] = k < toff[t + 1] - toff[t] ? th[toff[t] + k] : 0xffffffffu;
   }
+  uint32_t* list = ws.candidates + size_t(e) * ws.cap.cells;
+  sl(n, a, b);
+  for (uint32_t j = a + threadIdx.x; j < b; j += T) list[j] = sIdx[j];
+  // the loose-track count of pg_event_counts (the last writer of the quality
+  // codes, the triplet cleaner, has finished)
+  if (r == 0 && threadIdx.x == 0) ws.ev[e].nLoose = nLoose;
+}
+static_assert(kResultTracks <= PF_MAX_DOUBLETS_PARAM, "the loose tuples' list fits the candidates' place");
+
+// What the vertex finder adds: the tracks' vertices, the vertices and the header.
+__global__ void __launch_bounds__(512) kPackVertices(Workspace ws, uint8_t* out) {
+  const uint32_t e = blockIdx.x, T = blockDim.x;
+  const EventCounters* c = ws.ev + e;
+  uint8_t* base = out + size_t(e) * kResultStride;
+  const uint32_t bins = ws.cap.tuples;
+  const uint32_t* toff = ws.tupleOff + size_t(e) * (bins + 1);
+  const int16_t* idv = ws.idv + size_t(e) * bins;
+  const uint32_t* list = ws.candidates + size_t(e) * ws.cap.cells;
+  const uint32_t guard = c->apcM >= bins ? bins - 1 : c->nTuples;
+  const uint32_t nLoose = c->nLoose, n = min(nLoose, kResultTracks);
   const bool hasVtx = c->nVertices > 0;
-  w32 = reinterpret_cast<uint32_t*>(base + kResOffVertex);
-  sl((n + 1) / 2, a, b);
-  for (uint32_t w = a + threadIdx.x; w < b; w += T)
-    w32[w] = packHalves(w, n, [&](uint32_t i) { return hasVtx ? uint32_t(uint16_t(ws.idv[tb + sIdx[i]])) : 0xffffu; });
+  uint32_t* w32 = reinterpret_cast<uint32_t*>(base + kResOffVertex);
+  for (uint32_t w = threadIdx.x; w < (n + 1) / 2; w += T)
+    w32[w] = packHalves(w, n, [&](uint32_t i) { return hasVtx ? uint32_t(uint16_t(idv[list[i]])) : 0xffffu; });
   const uint32_t nv = min(c->nVertices, uint32_t(kMaxVtx));
   const size_t vb = size_t(e) * kMaxVtx;
   ResultVertices vtx = resultVertices(base);
-  sl(nv, a, b);
-  for (uint32_t v = a + threadIdx.x; v < b; v += T) {
+  for (uint32_t v = threadIdx.x; v < nv; v += T) {
     vtx.zv[v] = ws.zv[vb + v];
     vtx.wv[v] = ws.wv[vb + v];
     vtx.chi2[v] = ws.vchi2[vb + v];
@@ -160,10 +181,9 @@ __global__ void __launch_bounds__(512) kPackResults(Workspace ws, uint8_t* out) 
     vtx.ndof[v] = ws.ndof[vb + v];
   }
   w32 = reinterpret_cast<uint32_t*>(base + kResOffSortInd);
-  sl((nv + 1) / 2, a, b);
-  for (uint32_t w = a + threadIdx.x; w < b; w += T)
+  for (uint32_t w = threadIdx.x; w < (nv + 1) / 2; w += T)
     w32[w] = packHalves(w, nv, [&](uint32_t i) { return uint32_t(ws.sortInd[vb + i]); });
-  if (r == 0 && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     ResultHeader h{};
     h.nTracks = n;
     h.nLooseAll = nLoose;
@@ -180,9 +200,6 @@ __global__ void __launch_bounds__(512) kPackResults(Workspace ws, uint8_t* out) 
     h.nearCA = c->nearCA;
     h.nearQuality = c->nearQuality;
     *reinterpret_cast<ResultHeader*>(base) = h;
-    // the loose-track count of pg_event_counts (the last writer of the
-    // quality codes, the triplet cleaner, has finished)
-    ws.ev[e].nLoose = nLoose;
   }
 }
 
@@ -192,20 +209,35 @@ void launchSetInput(Workspace& ws, const uint32_t* words, const uint8_t* fedIds,
   PG_PROBED("kSetInput", s, kSetInput<<<1, 1, 0, s>>>(ws.input, words, fedIds));
 }
 
-void launchPack(Workspace& ws, uint32_t nEvents, uint8_t* out, cudaStream_t s) {
+cudaError_t runVerticesAndPack(Workspace& ws, uint32_t nEvents, int vertexAlgo, uint8_t* out, cudaStream_t stream,
+                               const SideStream& side) {
   // opt in to more than 48 KB of dynamic shared memory, once per device
   static std::atomic<uint64_t> ready{0};
   int dev = 0;
   cudaGetDevice(&dev);
   const uint64_t bit = uint64_t(1) << (dev & 63);
+  cudaError_t e = cudaSuccess;
   if (!(ready.load() & bit)) {
-    if (cudaFuncSetAttribute(kPackResults, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPackSmemBytes)) ==
-        cudaSuccess)
-      ready.fetch_or(bit);
+    e = cudaFuncSetAttribute(kPackTracks, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPackSmemBytes));
+    if (e != cudaSuccess) return e;
+    ready.fetch_or(bit);
   }
+  // The track packing is bound by the bus to the host and the vertex finder by
+  // the chain of its steps on a few SMs: side by side they take the longer of
+  // the two times (one PU50 event: 24 and 50 us, 64 of them: 300 and 90 us).
+  if ((e = cudaEventRecord(side.fork, stream)) != cudaSuccess) return e;
+  if ((e = cudaStreamWaitEvent(side.stream, side.fork, 0)) != cudaSuccess) return e;
   const uint32_t P = nEvents <= kClusterMaxEvents ? kPackCtas : 1;
-  // a failed launch is reported by the stream's next error check
-  PG_PROBED("kPackResults", s, (void)launchClustered(kPackResults, P, nEvents, 512, kPackSmemBytes, s, ws, out));
+  PG_PROBED("kPackTracks", side.stream,
+            e = launchClustered(kPackTracks, P, nEvents, 512, kPackSmemBytes, side.stream, ws, out));
+  // the side stream is joined whatever fails, so that a capture ends cleanly
+  const cudaError_t ev = runVertices(ws, nEvents, stream, vertexAlgo);
+  const cudaError_t er = cudaEventRecord(side.join, side.stream);
+  const cudaError_t ew = er == cudaSuccess ? cudaStreamWaitEvent(stream, side.join, 0) : er;
+  for (cudaError_t x : {e, ev, ew})
+    if (x != cudaSuccess) return x;
+  PG_PROBED("kPackVertices", stream, kPackVertices<<<nEvents, 512, 0, stream>>>(ws, out));
+  return cudaGetLastError();
 }
 
 }  // namespace pixgpu

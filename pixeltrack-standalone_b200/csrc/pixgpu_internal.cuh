@@ -398,9 +398,11 @@ cudaError_t launchClustered(void (*k)(KArgs...), uint32_t x, uint32_t nEvents, u
 // Runs the whole chain on events [0, nEvents) of ws, on `stream`.  The
 // word/fedId/offset inputs must already be in ws.  Returns a CUDA error code.
 // riemann: the Riemann fit in place of the broken-line fit (useRiemannFit);
-// vertexAlgo: the vertex clusterer (runVertices)
-cudaError_t runChain(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStream_t stream, bool riemann = false,
-                     int vertexAlgo = 0);
+// vertexAlgo: the vertex clusterer (runVertices); out: the results' host
+// memory (device address)
+struct SideStream;
+cudaError_t runChain(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStream_t stream, const SideStream& side,
+                     uint8_t* out, bool riemann = false, int vertexAlgo = 0);
 // Individual stages (used by runChain and by the stage-level tests)
 cudaError_t runLocal(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStream_t stream);
 // countModules + findClus + clusterChargeCut on digis already in ws
@@ -422,7 +424,16 @@ inline uint32_t tunedGrid(const Workspace& ws, TuneId id, uint32_t base) {
 
 // device FED scan: wordOffsets, words and fedIds of the batch from ws.scan
 void launchFedScan(Workspace& ws, uint32_t nEvents, cudaStream_t stream);
-void launchPack(Workspace& ws, uint32_t nEvents, uint8_t* out, cudaStream_t s);
+// a stream that runs beside a slot's stream between two events, always joined
+// to it before the batch ends
+struct SideStream {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+// the vertex finder on `stream`, with the packing of the tracks beside it on the
+// side stream, then the packing of the vertices
+cudaError_t runVerticesAndPack(Workspace& ws, uint32_t nEvents, int vertexAlgo, uint8_t* out, cudaStream_t stream,
+                               const SideStream& side);
 
 // batched segmented exclusive scan: out[e*stride + i] = sum_{k<i} in[e*stride + k]
 // for i <= n_e, where n_e = lenPtr[e*lenStride] (device) or maxLen when lenPtr is

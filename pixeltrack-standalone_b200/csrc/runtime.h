@@ -30,6 +30,7 @@ struct Slot {
   void* dmem = nullptr;
   Workspace ws{};
   cudaStream_t stream = nullptr;
+  SideStream side;                 // the part of a batch that runs beside the stream
   cudaEvent_t done = nullptr;      // end of the chain + result packing
   cudaEvent_t gathered = nullptr;  // pooled inputs copied out of the pool
   uint32_t* hWords = nullptr;      // pinned staging of unpacked words
