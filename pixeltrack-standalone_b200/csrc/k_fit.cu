@@ -433,119 +433,124 @@ __device__ __forceinline__ uint32_t fitBinPrefix(const Workspace& ws, uint32_t n
   return pre[nEvents];
 }
 
-// one thread per (tuple of the multiplicity bin nh); fits the first N hits
-template <int N, int kMode = kFitBrokenLine>
-__device__ __forceinline__ void blFitBin(const DeviceES& es, const Workspace& ws, uint32_t nh, uint32_t nEvents,
-                                         uint32_t* pre, uint32_t* scanSh) {
+// one thread per tuple of the multiplicity bin nh, flat items [g0, g0 +
+// blockDim.x) of total; fits the first N hits
+template <int N, int kMode>
+__device__ __forceinline__ void fitTile(const DeviceES& es, const Workspace& ws, uint32_t nh, uint32_t nEvents,
+                                        const uint32_t* pre, uint32_t g0, uint32_t total) {
   extern __shared__ double tile[];  // the threads' inputs (FitTile)
-  const uint32_t total = fitBinPrefix(ws, nh, nEvents, pre, scanSh);
   const double B = double(float(0.0114256972711507));
-  for (uint32_t g0 = blockIdx.x * blockDim.x; g0 < total; g0 += gridDim.x * blockDim.x) {
-    // the block fits in step (PG_FIT_PHASE): threads past the end repeat the last item
-    const bool live = g0 + threadIdx.x < total;
-    const uint32_t g = min(g0 + threadIdx.x, total - 1);
-    // the event of flat item g: the last e with pre[e] <= g (empty events skipped)
-    uint32_t lo = 0, hi = nEvents;
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (pre[mid] <= g)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    const uint32_t e = lo, k = g - pre[lo];
-    const uint32_t start = ws.tmOff[size_t(e) * 16 + 8 + nh];
-    const uint32_t* bins = ws.tmBins + size_t(e) * ws.cap.tuples;
-    const uint32_t* toff = ws.tupleOff + size_t(e) * (ws.cap.tuples + 1);
-    const uint32_t* th = ws.tupleHits + size_t(e) * ws.cap.tupleHits();
-    const size_t hb = size_t(e) * ws.cap.hits;
-    const size_t tb = size_t(e) * ws.cap.tuples;
-    uint32_t tkid = bins[start + k];
-    const uint32_t* hid = th + toff[tkid];
-    double* H = reinterpret_cast<double*>(tile) + threadIdx.x * FitTile<N>::kHitStride;
-    float* ge = reinterpret_cast<float*>(tile + blockDim.x * FitTile<N>::kHitStride) + threadIdx.x * FitTile<N>::kGeStride;
+  // the block fits in step (PG_FIT_PHASE): threads past the end repeat the last item
+  const bool live = g0 + threadIdx.x < total;
+  const uint32_t g = min(g0 + threadIdx.x, total - 1);
+  // the event of flat item g: the last e with pre[e] <= g (empty events skipped)
+  uint32_t lo = 0, hi = nEvents;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (pre[mid] <= g)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  const uint32_t e = lo, k = g - pre[lo];
+  const uint32_t start = ws.tmOff[size_t(e) * 16 + 8 + nh];
+  const uint32_t* bins = ws.tmBins + size_t(e) * ws.cap.tuples;
+  const uint32_t* toff = ws.tupleOff + size_t(e) * (ws.cap.tuples + 1);
+  const uint32_t* th = ws.tupleHits + size_t(e) * ws.cap.tupleHits();
+  const size_t hb = size_t(e) * ws.cap.hits;
+  const size_t tb = size_t(e) * ws.cap.tuples;
+  uint32_t tkid = bins[start + k];
+  const uint32_t* hid = th + toff[tkid];
+  double* H = reinterpret_cast<double*>(tile) + threadIdx.x * FitTile<N>::kHitStride;
+  float* ge = reinterpret_cast<float*>(tile + blockDim.x * FitTile<N>::kHitStride) + threadIdx.x * FitTile<N>::kGeStride;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    uint32_t hit = hid[i];
+    const PfFrame& f = es.det[ws.detInd[hb + hit]].frame;
+    float cxx = ws.xerr[hb + hit], cxy = 0, cyy = ws.yerr[hb + hit];
+    float* gl = ge + 6 * i;
+    gl[0] = f.R11 * (f.R11 * cxx + f.R21 * cxy) + f.R21 * (f.R11 * cxy + f.R21 * cyy);
+    gl[1] = f.R11 * (f.R12 * cxx + f.R22 * cxy) + f.R21 * (f.R12 * cxy + f.R22 * cyy);
+    gl[2] = f.R12 * (f.R12 * cxx + f.R22 * cxy) + f.R22 * (f.R12 * cxy + f.R22 * cyy);
+    gl[3] = f.R11 * (f.R13 * cxx + f.R23 * cxy) + f.R21 * (f.R13 * cxy + f.R23 * cyy);
+    gl[4] = f.R12 * (f.R13 * cxx + f.R23 * cxy) + f.R22 * (f.R13 * cxy + f.R23 * cyy);
+    gl[5] = f.R13 * (f.R13 * cxx + f.R23 * cxy) + f.R23 * (f.R13 * cxy + f.R23 * cyy);
+    H[3 * i + 0] = ws.xg[hb + hit];
+    H[3 * i + 1] = ws.yg[hb + hit];
+    H[3 * i + 2] = ws.zg[hb + hit];
+  }
+  FitOut o;
+  if constexpr (kMode == kFitRiemann) {
+    rfFit<N, double>(H, ge, B, o);
+  } else if constexpr (kMode == kFitRiemannMixed) {
+    rfFit<N, float>(H, ge, B, o);
+  } else if constexpr (kMode == kFitBrokenLineMixed) {
+    // the mixed fit takes single-precision hits relative to the first one
+    // and the first hit in double precision (k_fit_mixed.cuh)
+    float Hf[3 * N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      uint32_t hit = hid[i];
-      const PfFrame& f = es.det[ws.detInd[hb + hit]].frame;
-      float cxx = ws.xerr[hb + hit], cxy = 0, cyy = ws.yerr[hb + hit];
-      float* gl = ge + 6 * i;
-      gl[0] = f.R11 * (f.R11 * cxx + f.R21 * cxy) + f.R21 * (f.R11 * cxy + f.R21 * cyy);
-      gl[1] = f.R11 * (f.R12 * cxx + f.R22 * cxy) + f.R21 * (f.R12 * cxy + f.R22 * cyy);
-      gl[2] = f.R12 * (f.R12 * cxx + f.R22 * cxy) + f.R22 * (f.R12 * cxy + f.R22 * cyy);
-      gl[3] = f.R11 * (f.R13 * cxx + f.R23 * cxy) + f.R21 * (f.R13 * cxy + f.R23 * cyy);
-      gl[4] = f.R12 * (f.R13 * cxx + f.R23 * cxy) + f.R22 * (f.R13 * cxy + f.R23 * cyy);
-      gl[5] = f.R13 * (f.R13 * cxx + f.R23 * cxy) + f.R23 * (f.R13 * cxy + f.R23 * cyy);
-      H[3 * i + 0] = ws.xg[hb + hit];
-      H[3 * i + 1] = ws.yg[hb + hit];
-      H[3 * i + 2] = ws.zg[hb + hit];
+      Hf[3 * i + 0] = float(H[3 * i + 0] - H[0]);
+      Hf[3 * i + 1] = float(H[3 * i + 1] - H[1]);
+      Hf[3 * i + 2] = float(H[3 * i + 2]);
     }
-    FitOut o;
-    if constexpr (kMode == kFitRiemann) {
-      rfFit<N, double>(H, ge, B, o);
-    } else if constexpr (kMode == kFitRiemannMixed) {
-      rfFit<N, float>(H, ge, B, o);
-    } else if constexpr (kMode == kFitBrokenLineMixed) {
-      // the mixed fit takes single-precision hits relative to the first one
-      // and the first hit in double precision (k_fit_mixed.cuh)
-      float Hf[3 * N];
+    blFitMixed<N>(Hf, ge, H[0], H[1], float(B), B, o);
+  } else {
+    blFit<N>(H, ge, B, o);
+  }
+  if (!live) return;
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        Hf[3 * i + 0] = float(H[3 * i + 0] - H[0]);
-        Hf[3 * i + 1] = float(H[3 * i + 1] - H[1]);
-        Hf[3 * i + 2] = float(H[3 * i + 2]);
-      }
-      blFitMixed<N>(Hf, ge, H[0], H[1], float(B), B, o);
+  for (int j = 0; j < 5; ++j) ws.state[tb * 5 + size_t(tkid) * 5 + j] = o.state[j];
+#pragma unroll
+  for (int j = 0; j < 15; ++j) ws.cov[tb * 15 + size_t(tkid) * 15 + j] = o.cov[j];
+  ws.pt[tb + tkid] = o.pt;
+  ws.eta[tb + tkid] = o.eta;
+  ws.chi2[tb + tkid] = o.chi2;
+}
+
+// The three multiplicity bins (3-hit tuples, 4-hit tuples, 5-hit tuples
+// fitted on their first 4 hits) in one launch of as many blocks as the SMs
+// hold, which take the batch's tuples in tiles of a block, the dearer bins
+// first.  The number of tuples is not known on the host, and a grid sized for
+// the usual event left the SMs to one block each on a heavy one (two PU180
+// events: 222 blocks, 374 us), while a larger grid costs a light one its idle blocks.
+template <int kMode>
+__device__ __forceinline__ void fitBins(const DeviceES& es, const Workspace& ws, uint32_t nEvents) {
+  __shared__ uint32_t pre[3][kFlatMaxEvents + 1], scanSh[33];
+  uint32_t total[3], tiles[3];
+#pragma unroll
+  for (uint32_t b = 0; b < 3; ++b) {
+    total[b] = fitBinPrefix(ws, 3 + b, nEvents, pre[b], scanSh);
+    tiles[b] = (total[b] + blockDim.x - 1) / blockDim.x;
+  }
+  for (uint32_t t = blockIdx.x; t < tiles[0] + tiles[1] + tiles[2]; t += gridDim.x) {
+    if (t < tiles[2] + tiles[1]) {
+      const uint32_t b = t < tiles[2] ? 2u : 1u, k = b == 2 ? t : t - tiles[2];
+      fitTile<4, kMode>(es, ws, 3 + b, nEvents, pre[b], k * blockDim.x, b == 2 ? total[2] : total[1]);
     } else {
-      blFit<N>(H, ge, B, o);
+      fitTile<3, kMode>(es, ws, 3, nEvents, pre[0], (t - tiles[2] - tiles[1]) * blockDim.x, total[0]);
     }
-    if (!live) continue;
-#pragma unroll
-    for (int j = 0; j < 5; ++j) ws.state[tb * 5 + size_t(tkid) * 5 + j] = o.state[j];
-#pragma unroll
-    for (int j = 0; j < 15; ++j) ws.cov[tb * 15 + size_t(tkid) * 15 + j] = o.cov[j];
-    ws.pt[tb + tkid] = o.pt;
-    ws.eta[tb + tkid] = o.eta;
-    ws.chi2[tb + tkid] = o.chi2;
   }
 }
 
-// the three multiplicity bins in one launch: blockIdx.z = 0, 1, 2 fits the
-// 3-hit tuples, the 4-hit tuples and the first 4 hits of the 5-hit tuples
 __global__ void __launch_bounds__(kFitBlock, 2) kBLFit(DeviceES es, Workspace ws, uint32_t nEvents) {
-  __shared__ uint32_t pre[kFlatMaxEvents + 1], scanSh[33];
-  if (blockIdx.z == 0)
-    blFitBin<3>(es, ws, 3, nEvents, pre, scanSh);
-  else
-    blFitBin<4>(es, ws, 3 + blockIdx.z, nEvents, pre, scanSh);
+  fitBins<kFitBrokenLine>(es, ws, nEvents);
 }
 
 // the same bins through the Riemann fit (useRiemannFit,
 // CAHitNtupletGeneratorOnGPU.cc:116-120; RiemannFitOnGPU.cc:3-110)
 __global__ void __launch_bounds__(kRiemannBlock, 4) kRiemannFit(DeviceES es, Workspace ws, uint32_t nEvents) {
-  __shared__ uint32_t pre[kFlatMaxEvents + 1], scanSh[33];
-  if (blockIdx.z == 0)
-    blFitBin<3, kFitRiemann>(es, ws, 3, nEvents, pre, scanSh);
-  else
-    blFitBin<4, kFitRiemann>(es, ws, 3 + blockIdx.z, nEvents, pre, scanSh);
+  fitBins<kFitRiemann>(es, ws, nEvents);
 }
 
 // the mixed-precision variants of both fits inside the chain (pg_config
 // mixed_fit): a precision choice beside the reference's FP64 fits, whose
 // effect on the chain's quality codes and vertices is measured against them
 __global__ void __launch_bounds__(kFitBlock, 2) kBLFitMixed(DeviceES es, Workspace ws, uint32_t nEvents) {
-  __shared__ uint32_t pre[kFlatMaxEvents + 1], scanSh[33];
-  if (blockIdx.z == 0)
-    blFitBin<3, kFitBrokenLineMixed>(es, ws, 3, nEvents, pre, scanSh);
-  else
-    blFitBin<4, kFitBrokenLineMixed>(es, ws, 3 + blockIdx.z, nEvents, pre, scanSh);
+  fitBins<kFitBrokenLineMixed>(es, ws, nEvents);
 }
 __global__ void __launch_bounds__(kRiemannBlock, 4) kRiemannFitMixed(DeviceES es, Workspace ws, uint32_t nEvents) {
-  __shared__ uint32_t pre[kFlatMaxEvents + 1], scanSh[33];
-  if (blockIdx.z == 0)
-    blFitBin<3, kFitRiemannMixed>(es, ws, 3, nEvents, pre, scanSh);
-  else
-    blFitBin<4, kFitRiemannMixed>(es, ws, 3 + blockIdx.z, nEvents, pre, scanSh);
+  fitBins<kFitRiemannMixed>(es, ws, nEvents);
 }
 
 template <int kBytes>
@@ -660,7 +665,7 @@ __global__ void __launch_bounds__(kRiemannBlock, 4) kRiemannFitDirect(uint32_t n
 // memory (up to 53 KB, above the default limit: opted in once per kernel and device)
 template <typename... KArgs, typename... Args>
 static cudaError_t launchFit(void (*k)(KArgs...), std::atomic<uint64_t>& configured, uint32_t most, uint32_t grid,
-                             uint32_t bins, uint32_t block, uint32_t tupleBytes, cudaStream_t stream, Args... args) {
+                             uint32_t block, uint32_t tupleBytes, cudaStream_t stream, Args... args) {
   int dev = 0;
   cudaGetDevice(&dev);
   const uint64_t bit = uint64_t(1) << (dev & 63);
@@ -669,7 +674,7 @@ static cudaError_t launchFit(void (*k)(KArgs...), std::atomic<uint64_t>& configu
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }
-  k<<<dim3(grid, 1, bins), block, size_t(block) * tupleBytes, stream>>>(args...);
+  k<<<grid, block, size_t(block) * tupleBytes, stream>>>(args...);
   return cudaGetLastError();
 }
 
@@ -677,16 +682,15 @@ cudaError_t runFits(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStr
   const uint32_t gx = nEvents >= 32 ? 8 : (nEvents >= 8 ? 32 : 148);
   dim3 g(gx, nEvents);
   PG_PROBED("kFitZero", stream, kFitZero<<<dim3(tunedGrid(ws, kTuneFitZero, g.x), nEvents), 256, 0, stream>>>(ws));
-  // FP64-bound: enough warps per SM to cover the double-precision latency
-  const uint32_t fx = nEvents >= 32 ? 16 : (nEvents >= 8 ? 64 : 296);
-  // one flat grid over the batch's tuples (z: the multiplicity bin), as many
-  // blocks of 128 as a grid row per event would have
-  const uint32_t fb = riemann ? kRiemannBlock : kFitBlock;
-  const uint32_t fg = (tunedGrid(ws, kTuneFit, fx) * nEvents * 128 + fb - 1) / fb;
+  // one wave of blocks of 512 threads per SM; a few events' tuples (a PU50 event
+  // has 10.6k) go in tiles of 64, over all SMs.  The launch table does not scale
+  // this grid: it follows from the SMs alone.
+  const uint32_t most = riemann ? kRiemannBlock : kFitBlock;
+  const uint32_t fb = nEvents <= 4 ? 64u : most, fg = 148 * (512 / fb);
   static std::atomic<uint64_t> configured[4];
   cudaError_t le = cudaSuccess;
   auto launch = [&](int which, auto kernel) {
-    le = launchFit(kernel, configured[which], fb, fg, 3, fb, FitTile<4>::kBytes, stream, es, ws, nEvents);
+    le = launchFit(kernel, configured[which], most, fg, fb, FitTile<4>::kBytes, stream, es, ws, nEvents);
   };
   if (riemann && ws.ca.mixedFit)
     PG_PROBED("kRiemannFitMixed", stream, launch(0, kRiemannFitMixed));
@@ -716,7 +720,7 @@ static cudaError_t launchDirect(void (*k)(KArgs...), const char* name, std::atom
   const uint32_t fb = directBlock(n, most);
   cudaError_t e = cudaSuccess;
   PG_PROBED(name, stream,
-            e = launchFit(k, configured, most, min((n - 1) / fb + 1, 148u * 16u), 1, fb, FitTile<N>::kBytes, stream, n,
+            e = launchFit(k, configured, most, min((n - 1) / fb + 1, 148u * 16u), fb, FitTile<N>::kBytes, stream, n,
                           hits, ge, B, state, cov, pt, eta, chi2));
   return e;
 }
