@@ -428,18 +428,34 @@ __global__ void kOuterHitFill(Workspace ws) {
 
 // ------------------------------------------------------------------ connect
 
+// The float quantities of GPUCACell::areAlignedRZ, as the serial build forms
+// them: the radial distance of the outermost hits, their squared distance,
+// twice the triangle's area.
+struct RZTriangle {
+  float radiusDiff, distance2, area;
+};
+__device__ __forceinline__ RZTriangle rzTriangle(float r1, float z1, float ri, float zi, float ro, float zo) {
+  RZTriangle t;
+  t.radiusDiff = fabsf(r1 - ro);
+  t.distance2 = t.radiusDiff * t.radiusDiff + (z1 - zo) * (z1 - zo);
+  t.area = z1 * (ri - ro) + zi * (ro - r1) + zo * (r1 - ri);
+  return t;
+}
+
 // GPUCACell::areAlignedRZ, single-precision part: false only for pairs that
-// fail the cut by a margin far above rounding (the squared inequality in
-// float with a relative margin of 1e-4; NaN operands, and right-hand sides
-// small enough for the squares to lose precision as subnormals, pass on to
-// the exact test)
+// fail the cut by a margin far above rounding.  The cut |area| pMin sqrt(d2) <=
+// thetaCut d2 rd, squared and divided by d2, is area^2 pMin^2 <= thetaCut^2
+// d2 rd^2; cutScale (rzCutScale) is pMin^2 / thetaCut^2 with a relative margin
+// of 1e-4.  NaN operands, and products small enough to lose precision as
+// subnormals, pass on to the exact test.
+__device__ __forceinline__ float rzCutScale(float thetaCut) {
+  return kPtMin * kPtMin / (1.0001f * thetaCut * thetaCut);
+}
 __device__ __forceinline__ bool alignedRZMaybe(float r1, float z1, float ri, float zi, float ro, float zo,
-                                               float thetaCut) {
-  float radius_diff = fabsf(r1 - ro);
-  float distance_13_squared = radius_diff * radius_diff + (z1 - zo) * (z1 - zo);
-  const float area = z1 * (ri - ro) + zi * (ro - r1) + zo * (r1 - ri);
-  const float rhs = thetaCut * distance_13_squared * radius_diff;
-  return !(rhs > 1e-15f && area * area * (kPtMin * kPtMin) * distance_13_squared > 1.0001f * rhs * rhs);
+                                               float cutScale) {
+  const RZTriangle t = rzTriangle(r1, z1, ri, zi, ro, zo);
+  const float reach = t.radiusDiff * t.radiusDiff * t.distance2;
+  return !(reach > 1e-25f && t.area * t.area * cutScale > reach);
 }
 
 // GPUCACell::areAlignedRZ: fabs(float) binds to the double overload in the
@@ -448,13 +464,11 @@ __device__ __forceinline__ bool alignedRZMaybe(float r1, float z1, float ri, flo
 // not counted as near it.
 __device__ __forceinline__ bool alignedRZ(float r1, float z1, float ri, float zi, float ro, float zo, float thetaCut,
                                           uint32_t& near) {
-  if (!alignedRZMaybe(r1, z1, ri, zi, ro, zo, thetaCut)) return false;
-  float radius_diff = fabsf(r1 - ro);
-  float distance_13_squared = radius_diff * radius_diff + (z1 - zo) * (z1 - zo);
-  const float area = z1 * (ri - ro) + zi * (ro - r1) + zo * (r1 - ri);
-  const float rhs = thetaCut * distance_13_squared * radius_diff;
+  const RZTriangle t = rzTriangle(r1, z1, ri, zi, ro, zo);
+  const float distance_13_squared = t.distance2;
+  const float rhs = thetaCut * distance_13_squared * t.radiusDiff;
   float pMin = kPtMin * sqrtf(distance_13_squared);
-  double lhs = fabs(double(area));
+  double lhs = fabs(double(t.area));
   near += cutNear(lhs * double(pMin), double(rhs));
   return lhs * double(pMin) <= double(rhs);
 }
@@ -588,7 +602,7 @@ __global__ void __launch_bounds__(kConnectWarps * 32, 5) kConnect(Workspace ws, 
     // cut), so that the warp's loads for 32 slots overlap
     const uint32_t jl = w + (r0 + lane) * S;
     uint32_t myBase = 0, myEnd = 0, myOb = 0, myM = 0, myH = 0;
-    float myRi = 0.f, myZi = 0.f, myTheta = 0.f, myInvM = 0.f;
+    float myRi = 0.f, myZi = 0.f, myScale = 0.f, myInvM = 0.f;
     if (jl < ntot) {
       myBase = joff[jl];
       myEnd = min(joff[jl + 1], nCells);
@@ -598,13 +612,7 @@ __global__ void __launch_bounds__(kConnectWarps * 32, 5) kConnect(Workspace ws, 
         myM = min(ohOff[myH + 1] - myOb, uint32_t(PF_MAX_CELLS_PER_HIT));
         myRi = hh.rg[myH];
         myZi = hh.zg[myH];
-        myTheta = hh.detInd[myH] < 1184 ? kThetaCutBarrel : kThetaCutForward;
-        // the slot's (cell, candidate) pairs are enumerated flat, 32 at a
-        // time: pair f is cell f / m of a chunk and candidate f % m, so only
-        // the last step of a chunk leaves lanes idle.  f < 32 * 128, so the
-        // quotient from the single-precision reciprocal is exact (the error,
-        // below 2^-11, is far under the 0.5 / m that (f + 0.5) / m keeps
-        // from an integer).
+        myScale = rzCutScale(hh.detInd[myH] < 1184 ? kThetaCutBarrel : kThetaCutForward);
         if (myM > 0) myInvM = 1.f / float(myM);
       }
     }
@@ -618,8 +626,16 @@ __global__ void __launch_bounds__(kConnectWarps * 32, 5) kConnect(Workspace ws, 
       const uint32_t m = __shfl_sync(0xffffffffu, myM, l);
       const uint32_t h = __shfl_sync(0xffffffffu, myH, l);
       const float ri = __shfl_sync(0xffffffffu, myRi, l), zi = __shfl_sync(0xffffffffu, myZi, l);
-      const float thetaCut = __shfl_sync(0xffffffffu, myTheta, l);
+      const float cutScale = __shfl_sync(0xffffffffu, myScale, l);
+      // the slot's (cell, candidate) pairs are enumerated flat, 32 at a time:
+      // pair f is cell f / m of a chunk and candidate f % m, so only the last
+      // step of a chunk leaves lanes idle.  A lane's next pair is 32 further:
+      // 32 / m cells and 32 % m candidates (the quotients from the
+      // single-precision reciprocal are exact: its error is far under the
+      // 0.5 / m that (f + 0.5) / m keeps from an integer).
       const float invM = __shfl_sync(0xffffffffu, myInvM, l);
+      const uint32_t t32 = uint32_t(32.5f * invM), k32 = 32 - t32 * m;
+      const uint32_t t0 = uint32_t((float(lane) + 0.5f) * invM), k0 = lane - t0 * m;
       for (uint32_t c0 = base; c0 < end; c0 += 32) {
         const uint32_t nc = min(32u, end - c0);
         float sro = 0.f, szo = 0.f;
@@ -630,21 +646,27 @@ __global__ void __launch_bounds__(kConnectWarps * 32, 5) kConnect(Workspace ws, 
           szo = hh.zg[soh];
         }
         const uint32_t P = nc * m;
+        uint32_t t = t0, k = k0;
         for (uint32_t f0 = 0; f0 < P; f0 += 32) {
-          const uint32_t f = f0 + lane;
-          const bool valid = f < P;
-          const uint32_t t = valid ? uint32_t((float(f) + 0.5f) * invM) : 0u;
-          const uint32_t k = f - t * m;
+          const bool valid = f0 + lane < P;
           const float ro = __shfl_sync(0xffffffffu, sro, t), zo = __shfl_sync(0xffffffffu, szo, t);
           float4 r1 = make_float4(0.f, 0.f, 0.f, 0.f);
           if (valid) r1 = ohRec[ob + k];
-          const bool pass = valid && alignedRZMaybe(fabsf(r1.w), r1.z, ri, zi, ro, zo, thetaCut);
+          const bool pass = valid && alignedRZMaybe(fabsf(r1.w), r1.z, ri, zi, ro, zo, cutScale);
           const uint32_t mask = __ballot_sync(0xffffffffu, pass);
-          if (mask == 0) continue;
-          const uint32_t oh = __shfl_sync(0xffffffffu, soh, t);
-          if (pass) queue[(qTail + __popc(mask & lanemaskLt())) & (kConnectQueue - 1)] = make_uint4(ob + k, c0 + t, h, oh);
-          qTail += __popc(mask);
-          if (qTail - qHead >= 32) drain(32);
+          if (mask) {
+            const uint32_t oh = __shfl_sync(0xffffffffu, soh, t);
+            if (pass)
+              queue[(qTail + __popc(mask & lanemaskLt())) & (kConnectQueue - 1)] = make_uint4(ob + k, c0 + t, h, oh);
+            qTail += __popc(mask);
+            if (qTail - qHead >= 32) drain(32);
+          }
+          t += t32;
+          k += k32;
+          if (k >= m) {
+            k -= m;
+            ++t;
+          }
         }
       }
     }

@@ -415,10 +415,17 @@ cudaError_t runCleaners(Workspace& ws, uint32_t nEvents, cudaStream_t stream);
 
 // batch input descriptor and compact results (k_pack.cu)
 void launchSetInput(Workspace& ws, const uint32_t* words, const uint8_t* fedIds, cudaStream_t s);
-// grid x-extent of a tunable launch
+// Grid x-extent of a tunable launch.  Contexts whose doublet capacity is
+// raised serve events of very different sizes (the tables are tuned at PU50):
+// a batch ends with its heaviest events, whose share of the grid is what runs
+// then, so the shares are larger there (12 uneven PU20-200 events: kConnect
+// -141 us, kFishbone -108 us, the other CA kernels about -40 us each at four
+// times the grid; the doublet kernels, whose staging shares shrink with it,
+// gain at twice: -56 and -42 us).
 inline uint32_t tunedGrid(const Workspace& ws, TuneId id, uint32_t base) {
-  const int s = ws.tune.scale[id];
-  uint64_t g = s >= 0 ? uint64_t(base) << s : uint64_t(base) >> (-s);
+  const bool wide = ws.cap.cells > 2 * uint32_t(PF_MAX_DOUBLETS_PARAM);
+  const int s = ws.tune.scale[id] + (!wide ? 0 : id == kTuneDoubletCount || id == kTuneDoubletWrite ? 1 : 2);
+  const uint64_t g = s >= 0 ? uint64_t(base) << s : uint64_t(base) >> (-s);
   return uint32_t(g < 1 ? 1 : (g > 65535 ? 65535 : g));
 }
 
