@@ -702,37 +702,6 @@ __global__ void kEdgeScatter(Workspace ws, const uint32_t* edgeOc, const uint32_
   }
 }
 
-// cells with at least one CA link must fit the 65535-list pool of the reference.
-// The same pass clears the n-tuplet search's per-cell counts and lists the
-// cells with links: a tuple has at least two cells, so only they can start
-// one.  The list goes to startHitOff, which is free until the scan of the
-// start-hit counts writes it.
-__global__ void kNbrPool(Workspace ws) {
-  uint32_t e = blockIdx.y;
-  EventCounters* c = ws.ev + e;
-  uint32_t n = c->nCells;
-  const uint32_t* off = ws.nbrOff + size_t(e) * (ws.cap.cells + 1);
-  uint32_t* tc = ws.startTupleCount + size_t(e) * (ws.cap.cells + 1);
-  uint32_t* hc = ws.startHitCount + size_t(e) * (ws.cap.cells + 1);
-  uint32_t* linked = ws.startHitOff + size_t(e) * (ws.cap.cells + 1);
-  uint32_t local = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const bool has = off[i + 1] > off[i];
-    local += has ? 1u : 0u;
-    tc[i] = 0;
-    hc[i] = 0;
-    const uint32_t active = __activemask();
-    const uint32_t bal = __ballot_sync(active, has);
-    const uint32_t leader = __ffs(active) - 1;
-    uint32_t at = 0;
-    if (laneId() == leader && bal) at = atomicAdd(&c->nLinked, uint32_t(__popc(bal)));
-    at = __shfl_sync(active, at, leader);
-    if (has) linked[at + __popc(bal & lanemaskLt())] = i;
-  }
-  local = __reduce_add_sync(0xffffffffu, local);
-  if ((threadIdx.x & 31) == 0 && local) atomicAdd(&c->nNbrLists, local);
-}
-
 // ------------------------------------------------------------------ fishbone
 
 // gpuFishbone.h:21-90 (early fishbone), one warp per hit with >= 2 cells
@@ -1001,7 +970,8 @@ __device__ __forceinline__ bool isStartCell(const Workspace& ws, size_t cb, uint
 // The count pass stages every tuple it finds, so that the write pass is a
 // flat copy instead of a second search: the tuple's cells padded with ~0
 // (scratchA, 16-byte aligned), and its rank and first-hit offset among the
-// tuples of its start cell (scratchB).  Both regions are free between the CA
+// tuples of its start cell, with that cell's place in the list of linked
+// cells (scratchB).  Both regions are free between the CA
 // links and the duplicate rounds.  Records are appended in any order (one
 // atomic per group of lanes that find a tuple together); the write pass puts
 // each at its serial position, the start cell's scanned offsets plus its
@@ -1011,6 +981,7 @@ struct TupleStage {
   uint4* cells;
   uint32_t* rank;
   uint32_t* hit;
+  uint32_t* start;
   uint32_t cap;
 };
 __device__ __forceinline__ TupleStage tupleStage(const Workspace& ws, uint32_t e) {
@@ -1021,6 +992,7 @@ __device__ __forceinline__ TupleStage tupleStage(const Workspace& ws, uint32_t e
   t.cells = reinterpret_cast<uint4*>(a + pad);
   t.rank = ws.scratchB + size_t(e) * ws.cap.scratch;
   t.hit = t.rank + t.cap;
+  t.start = t.hit + t.cap;
   return t;
 }
 
@@ -1034,9 +1006,14 @@ __global__ void kNtupletCount(Workspace ws) {
   uint32_t* tc = ws.startTupleCount + size_t(e) * (ws.cap.cells + 1);
   uint32_t* hc = ws.startHitCount + size_t(e) * (ws.cap.cells + 1);
   const TupleStage st = tupleStage(ws, e);
-  // the cells with links (kNbrPool; the counts of all others are zero)
-  const uint32_t* linked = ws.startHitOff + size_t(e) * (ws.cap.cells + 1);
+  // The cells with links, ascending (listed by the scan of the links' counts):
+  // a tuple has at least two cells, so only they can start one.  The counts
+  // are kept by place in that list, so the scans that follow run over the
+  // linked cells (one in twenty at PU50) instead of all.
+  const uint32_t* linked = ws.candidates + size_t(e) * ws.cap.cells;
   const uint32_t nl = c->nLinked;
+  // the lists in use, with the reserved empty one (kMultiplicity checks the reference's pool)
+  if (blockIdx.x == 0 && threadIdx.x == 0) c->nNbrLists = nl + 1;
   for (uint32_t li = blockIdx.x * blockDim.x + threadIdx.x; li < nl; li += gridDim.x * blockDim.x) {
     const uint32_t idx = linked[li];
     uint32_t nt = 0, nh = 0;
@@ -1051,21 +1028,21 @@ __global__ void kNtupletCount(Workspace ws) {
                                    ncells > 3 ? cells[3] : ~0u);
           st.rank[s] = nt;
           st.hit[s] = nh;
+          st.start[s] = li;
         }
         ++nt;
         nh += uint32_t(ncells) + 1;
       });
       if (!ok) atomicOr(&c->flags, kFlagDeepTuple);
     }
-    tc[idx] = nt;
-    hc[idx] = nh;
+    tc[li] = nt;
+    hc[li] = nh;
   }
 }
 
 __global__ void kNtupletWrite(Workspace ws) {
   uint32_t e = blockIdx.y;
   EventCounters* c = ws.ev + e;
-  uint32_t n = c->nCells;
   size_t cb = size_t(e) * ws.cap.cells;
   const uint32_t* nbrOff = ws.nbrOff + size_t(e) * (ws.cap.cells + 1);
   const uint32_t* nbr = ws.nbr + size_t(e) * ws.cap.edges;
@@ -1080,9 +1057,10 @@ __global__ void kNtupletWrite(Workspace ws) {
   if (staged <= st.cap) {
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < staged; s += gridDim.x * blockDim.x) {
       const uint4 r = st.cells[s];
-      const uint32_t m = to[r.x] + st.rank[s];
+      const uint32_t li = st.start[s];
+      const uint32_t m = to[li] + st.rank[s];
       if (m >= ws.cap.tuples) continue;
-      const uint32_t off = ho[r.x] + st.hit[s];
+      const uint32_t off = ho[li] + st.hit[s];
       toff[m] = off;
       // the cells (at least two) and their hits; the per-event stride of
       // tcell is 4 * cap.tuples words on a 256-byte aligned base
@@ -1105,9 +1083,11 @@ __global__ void kNtupletWrite(Workspace ws) {
     }
     return;
   }
-  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
+  const uint32_t* linked = ws.candidates + size_t(e) * ws.cap.cells;
+  for (uint32_t li = blockIdx.x * blockDim.x + threadIdx.x; li < c->nLinked; li += gridDim.x * blockDim.x) {
+    const uint32_t idx = linked[li];
     if (!isStartCell(ws, cb, idx)) continue;
-    uint32_t m = to[idx], off = ho[idx];
+    uint32_t m = to[li], off = ho[li];
     if (m >= ws.cap.tuples) continue;
     dfsNtuplets(idx, ws.cellDoubletId + cb, nbrOff, nbr, ws.ca.minHits, [&](int ncells, const uint32_t* cells) {
       if (m < ws.cap.tuples) {
@@ -1708,19 +1688,19 @@ cudaError_t runCA(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStrea
   if (ws.ca.earlyFishbone)
     PG_PROBED("kZero", stream, kZero<<<dim3(gx, nEvents), 256, 0, stream>>>(ws.hitTouch, kHitCap, kHitCap, EVF(nHits)));
   PG_PROBED("kConnect", stream, kConnect<<<dim3(tunedGrid(ws, kTuneConnect, gx * 4), nEvents), kConnectWarps * 32, 0, stream>>>(ws, ws.scratchA, ws.scratchB));
-  segScan(ws, kScanNeighbours, ws.nbrCount, ws.nbrOff, kCellCap + 1, EVF(nCells), kCellCap, nullptr, 0, nEvents, stream,
-          true);
+  // (the linked cells' list stays in ws.candidates until kTrackPool)
+  segScanList(ws, kScanNeighbours, ws.nbrCount, ws.nbrOff, kScanLinked, ws.candidates, &ws.ev[0].nLinked, kCellCap + 1,
+              kCellCap, EVF(nCells), kCellCap, sizeof(EventCounters) / 4, nEvents, stream);
   PG_PROBED("kEdgeScatter", stream, kEdgeScatter<<<dim3(tunedGrid(ws, kTuneEdgeScatter, gx), nEvents), 256, 0, stream>>>(ws, ws.scratchA, ws.scratchB));
   sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.nbr, ws.cap.edges, ws.nbrOff, kCellCap + 1, EVF(nCells), 0, false,
                          min(ws.cap.edges, ws.cap.scratch), 1);
-  PG_PROBED("kNbrPool", stream, kNbrPool<<<dim3(tunedGrid(ws, kTuneNbrPool, gx), nEvents), 256, 0, stream>>>(ws));
   // ---- early fishbone
   if (ws.ca.earlyFishbone)
     PG_PROBED("kFishbone", stream, kFishbone<<<dim3(tunedGrid(ws, kTuneFishbone, gx * 2), nEvents), 256, 0, stream>>>(ws, false));
   // ---- n-tuplets: DFS count, scans, DFS write, finalize
   PG_PROBED("kNtupletCount", stream, kNtupletCount<<<dim3(tunedGrid(ws, kTuneNtupletCount, gx * 8), nEvents), 128, 0, stream>>>(ws));
   segScan2(ws, kScanStartTuples, ws.startTupleCount, ws.startTupleOff, &ws.ev[0].apcM, kScanStartHits, ws.startHitCount,
-           ws.startHitOff, &ws.ev[0].apcN, kCellCap + 1, EVF(nCells), kCellCap, sizeof(EventCounters) / 4, nEvents,
+           ws.startHitOff, &ws.ev[0].apcN, kCellCap + 1, EVF(nLinked), kCellCap, sizeof(EventCounters) / 4, nEvents,
            stream);
   PG_PROBED("kNtupletWrite", stream, kNtupletWrite<<<dim3(tunedGrid(ws, kTuneNtupletWrite, gx * 8), nEvents), 128, 0, stream>>>(ws));
   PG_PROBED("kTupleFinalize", stream, kTupleFinalize<<<dim3(32, nEvents), 1024, 0, stream>>>(ws));

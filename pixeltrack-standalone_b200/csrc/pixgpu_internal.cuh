@@ -188,6 +188,7 @@ enum ScanCall : uint32_t {
   kScanStartHits,
   kScanCellTracks,
   kScanHitTuples,
+  kScanLinked,
   kScanCalls
 };
 constexpr uint32_t kScanTile = 4096;  // elements per tile of the single-pass scan
@@ -291,6 +292,8 @@ struct Workspace {
   uint32_t* nbrOff;          // [maxEvents][cap.cells + 1]
   uint32_t* nbr;             // [maxEvents][cap.edges]
   // tuples
+  // tuples and their hits by starting cell, indexed by the cell's place in the
+  // list of cells with CA links
   uint32_t* startTupleCount; // [maxEvents][cap.cells + 1]
   uint32_t* startTupleOff;   // [maxEvents][cap.cells + 1]
   uint32_t* startHitCount;   // [maxEvents][cap.cells + 1]
@@ -451,6 +454,11 @@ cudaError_t runVerticesAndPack(Workspace& ws, uint32_t nEvents, int vertexAlgo, 
 void segScan(const Workspace& ws, ScanCall call, uint32_t* in, uint32_t* out, uint32_t stride,
              const uint32_t* lenPtr, uint32_t lenStride, uint32_t maxLen, uint32_t* totalPtr, uint32_t totalStride,
              uint32_t nEvents, cudaStream_t stream, bool zeroIn = false);
+// A scan of counts (in is left zero) that also lists the indices of the
+// nonzero ones, ascending, at list[e*listStride]; their number lands at listTotal.
+void segScanList(const Workspace& ws, ScanCall call, uint32_t* in, uint32_t* out, ScanCall listCall, uint32_t* list,
+                 uint32_t* listTotal, uint32_t stride, uint32_t listStride, const uint32_t* lenPtr, uint32_t lenStride,
+                 uint32_t maxLen, uint32_t totalStride, uint32_t nEvents, cudaStream_t stream);
 // Two such scans of arrays with the same lengths and stride in one launch.
 void segScan2(const Workspace& ws, ScanCall call0, uint32_t* in0, uint32_t* out0, uint32_t* total0, ScanCall call1,
               uint32_t* in1, uint32_t* out1, uint32_t* total1, uint32_t stride, const uint32_t* lenPtr,

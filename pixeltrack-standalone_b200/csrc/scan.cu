@@ -52,10 +52,12 @@ struct ScanArray {
   uint32_t call;    // ScanCall: state region
 };
 
-template <uint32_t kArrays>
+// kList: the second array is formed from the first, 1 for each nonzero count,
+// and its prefix places the indices of those in a1.out (stride listStride)
+template <uint32_t kArrays, bool kList = false>
 __global__ void __launch_bounds__(kScanThreads, 3)
     kScanOnePass(ScanArray a0, ScanArray a1, uint32_t stride, const uint32_t* lenPtr, uint32_t lenStride,
-                 uint32_t fixedLen, uint32_t totalStride, bool zeroIn, Workspace ws) {
+                 uint32_t fixedLen, uint32_t totalStride, bool zeroIn, uint32_t listStride, Workspace ws) {
   __shared__ uint32_t sh[kArrays][33];
   __shared__ uint32_t sTile, sPrefix[kArrays];
   const uint32_t e = blockIdx.y;
@@ -73,13 +75,21 @@ __global__ void __launch_bounds__(kScanThreads, 3)
     const uint32_t w0 = lo + warp * 32 * kScanPer + lane;
     uint32_t v[kArrays][kScanPer];
     uint32_t base[kArrays], tileTot[kArrays];
+    uint32_t nonzero = 0;  // kList: bit j, v[0][j] is a nonzero count
 #pragma unroll
-    for (uint32_t q = 0; q < kArrays; ++q) {
+    for (uint32_t q = 0; q < (kList ? 1u : kArrays); ++q) {
       const uint32_t* src = arr(q).in + size_t(e) * stride;
 #pragma unroll
       for (uint32_t j = 0; j < kScanPer; ++j) {
         const uint32_t i = w0 + j * 32;
         v[q][j] = i < hi ? src[i] : 0u;
+      }
+    }
+    if (kList) {
+#pragma unroll
+      for (uint32_t j = 0; j < kScanPer; ++j) {
+        v[kArrays - 1][j] = v[0][j] != 0 ? 1u : 0u;
+        nonzero |= v[kArrays - 1][j] << j;
       }
     }
 #pragma unroll
@@ -138,9 +148,17 @@ __global__ void __launch_bounds__(kScanThreads, 3)
     __syncthreads();
 #pragma unroll
     for (uint32_t q = 0; q < kArrays; ++q) {
+      const uint32_t carry = sPrefix[q] + base[q];
+      if (kList && q == 1) {
+        uint32_t* list = a1.out + size_t(e) * listStride;
+#pragma unroll
+        for (uint32_t j = 0; j < kScanPer; ++j)
+          if ((nonzero >> j) & 1u) list[carry + v[q][j]] = w0 + j * 32;
+        if (t == tiles - 1 && threadIdx.x == 0) a1.total[size_t(e) * totalStride] = sPrefix[q] + tileTot[q];
+        continue;
+      }
       uint32_t* src = arr(q).in + size_t(e) * stride;
       uint32_t* dst = arr(q).out + size_t(e) * stride;
-      const uint32_t carry = sPrefix[q] + base[q];
 #pragma unroll
       for (uint32_t j = 0; j < kScanPer; ++j) {
         const uint32_t i = w0 + j * 32;
@@ -174,7 +192,16 @@ void segScan(const Workspace& ws, ScanCall call, uint32_t* in, uint32_t* out, ui
   const ScanArray a{in, out, totalPtr, uint32_t(call)};
   PG_PROBED("kScanOnePass", stream,
             kScanOnePass<1><<<scanGrid(maxLen, nEvents), kScanThreads, 0, stream>>>(
-                a, a, stride, lenPtr, lenStride, maxLen, totalStride, zeroIn, ws));
+                a, a, stride, lenPtr, lenStride, maxLen, totalStride, zeroIn, 0u, ws));
+}
+
+void segScanList(const Workspace& ws, ScanCall call, uint32_t* in, uint32_t* out, ScanCall listCall, uint32_t* list,
+                 uint32_t* listTotal, uint32_t stride, uint32_t listStride, const uint32_t* lenPtr, uint32_t lenStride,
+                 uint32_t maxLen, uint32_t totalStride, uint32_t nEvents, cudaStream_t stream) {
+  const ScanArray a0{in, out, nullptr, uint32_t(call)}, a1{nullptr, list, listTotal, uint32_t(listCall)};
+  PG_PROBED("kScanOnePass", stream,
+            (kScanOnePass<2, true><<<scanGrid(maxLen, nEvents), kScanThreads, 0, stream>>>(
+                a0, a1, stride, lenPtr, lenStride, maxLen, totalStride, true, listStride, ws)));
 }
 
 void segScan2(const Workspace& ws, ScanCall call0, uint32_t* in0, uint32_t* out0, uint32_t* total0, ScanCall call1,
@@ -184,7 +211,7 @@ void segScan2(const Workspace& ws, ScanCall call0, uint32_t* in0, uint32_t* out0
   const ScanArray a0{in0, out0, total0, uint32_t(call0)}, a1{in1, out1, total1, uint32_t(call1)};
   PG_PROBED("kScanOnePass", stream,
             kScanOnePass<2><<<scanGrid(maxLen, nEvents), kScanThreads, 0, stream>>>(
-                a0, a1, stride, lenPtr, lenStride, maxLen, totalStride, zeroIn, ws));
+                a0, a1, stride, lenPtr, lenStride, maxLen, totalStride, zeroIn, 0u, ws));
 }
 
 }  // namespace pixgpu
