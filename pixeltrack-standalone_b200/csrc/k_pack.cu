@@ -127,25 +127,36 @@ __global__ void __launch_bounds__(512) kPackTracks(Workspace ws, uint8_t* out) {
     w32[w] = packBytes(w, n, [&](uint32_t i) { return toff[sIdx[i] + 1] - toff[sIdx[i]]; });
   w32 = reinterpret_cast<uint32_t*>(base + kResOffQuality);
   for (uint32_t w = a + threadIdx.x; w < b; w += T) w32[w] = packBytes(w, n, [&](uint32_t i) { return q[sIdx[i]]; });
-  float* f = reinterpret_cast<float*>(base + kResOffState);
-  sl(5 * n, a, b);
-  for (uint32_t j = a + threadIdx.x; j < b; j += T) f[j] = ws.state[tb * 5 + size_t(sIdx[j / 5]) * 5 + j % 5];
-  f = reinterpret_cast<float*>(base + kResOffCov);
-  sl(15 * n, a, b);
-  for (uint32_t j = a + threadIdx.x; j < b; j += T) f[j] = ws.cov[tb * 15 + size_t(sIdx[j / 15]) * 15 + j % 15];
+  // the arrays with several words per track: four words per thread and store
+  // (the last store's words past the end are zero)
+  auto quads = [&](size_t off, uint32_t len, auto&& word) {
+    uint4* q4 = reinterpret_cast<uint4*>(base + off);
+    sl((len + 3) / 4, a, b);
+    for (uint32_t w = a + threadIdx.x; w < b; w += T) {
+      uint32_t x[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) x[k] = 4 * w + k < len ? word(4 * w + k) : 0u;
+      q4[w] = make_uint4(x[0], x[1], x[2], x[3]);
+    }
+  };
+  static_assert(kResOffState % 16 == 0 && kResOffCov % 16 == 0 && kResOffHits % 16 == 0, "16-byte stores");
+  quads(kResOffState, 5 * n, [&](uint32_t j) {
+    return __float_as_uint(ws.state[tb * 5 + size_t(sIdx[j / 5]) * 5 + j % 5]);
+  });
+  quads(kResOffCov, 15 * n, [&](uint32_t j) {
+    return __float_as_uint(ws.cov[tb * 15 + size_t(sIdx[j / 15]) * 15 + j % 15]);
+  });
   sl(n, a, b);
-  f = reinterpret_cast<float*>(base + kResOffPt);
+  float* f = reinterpret_cast<float*>(base + kResOffPt);
   for (uint32_t j = a + threadIdx.x; j < b; j += T) f[j] = ws.pt[tb + sIdx[j]];
   f = reinterpret_cast<float*>(base + kResOffEta);
   for (uint32_t j = a + threadIdx.x; j < b; j += T) f[j] = ws.eta[tb + sIdx[j]];
   f = reinterpret_cast<float*>(base + kResOffChi2);
   for (uint32_t j = a + threadIdx.x; j < b; j += T) f[j] = ws.chi2[tb + sIdx[j]];
-  w32 = reinterpret_cast<uint32_t*>(base + kResOffHits);
-  sl(5 * n, a, b);
-  for (uint32_t i = a + threadIdx.x; i < b; i += T) {
+  quads(kResOffHits, 5 * n, [&](uint32_t i) {
     const uint32_t t = sIdx[i / 5], k = i % 5;
-    w32[i] = k < toff[t + 1] - toff[t] ? th[toff[t] + k] : 0xffffffffu;
-  }
+    return k < toff[t + 1] - toff[t] ? th[toff[t] + k] : 0xffffffffu;
+  });
   uint32_t* list = ws.candidates + size_t(e) * ws.cap.cells;
   sl(n, a, b);
   for (uint32_t j = a + threadIdx.x; j < b; j += T) list[j] = sIdx[j];
@@ -227,11 +238,14 @@ cudaError_t runVerticesAndPack(Workspace& ws, uint32_t nEvents, int vertexAlgo, 
   // the two times (one PU50 event: 24 and 50 us, 64 of them: 300 and 90 us).
   if ((e = cudaEventRecord(side.fork, stream)) != cudaSuccess) return e;
   if ((e = cudaStreamWaitEvent(side.stream, side.fork, 0)) != cudaSuccess) return e;
-  const uint32_t P = nEvents <= kClusterMaxEvents ? kPackCtas : 1;
+  // The vertex finder goes first: its clusters need whole SMs of one GPC, and
+  // waited for the packing's CTAs where those came first (8 PU50 events: 69 -> 80 us).
+  const cudaError_t ev = runVertices(ws, nEvents, stream, vertexAlgo);
+  // four CTAs per event keep the bus busy once there are a few events
+  const uint32_t P = nEvents <= 4 ? kPackCtas : (nEvents <= kClusterMaxEvents ? kPackCtas / 2 : 1);
   PG_PROBED("kPackTracks", side.stream,
             e = launchClustered(kPackTracks, P, nEvents, 512, kPackSmemBytes, side.stream, ws, out));
   // the side stream is joined whatever fails, so that a capture ends cleanly
-  const cudaError_t ev = runVertices(ws, nEvents, stream, vertexAlgo);
   const cudaError_t er = cudaEventRecord(side.join, side.stream);
   const cudaError_t ew = er == cudaSuccess ? cudaStreamWaitEvent(stream, side.join, 0) : er;
   for (cudaError_t x : {e, ev, ew})
