@@ -68,9 +68,20 @@ __device__ __forceinline__ HitsView hitsOf(const Workspace& ws, uint32_t e) {
 
 // ------------------------------------------------------------------ doublets
 
-__global__ void kDoubletSetup(Workspace ws, uint32_t nEvents) {
-  uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nEvents) return;
+// Clears the per-hit counters of the kernels to come (cells by outer hit, link
+// ends, tuples by hit) and sets up the event's doublet slots.
+__global__ void kHitArrays(Workspace ws) {
+  const uint32_t e = blockIdx.y;
+  const uint32_t n = min(ws.ev[e].nHits, ws.cap.hits);
+  uint32_t* oh = ws.ohCount + size_t(e) * (ws.cap.hits + 1);
+  uint32_t* h2t = ws.h2tCount + size_t(e) * (ws.cap.hits + 1);
+  uint32_t* touch = ws.hitTouch + size_t(e) * ws.cap.hits;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
+    oh[i] = 0;
+    h2t[i] = 0;
+    if (i < n) touch[i] = 0;
+  }
+  if (blockIdx.x != 0 || threadIdx.x != 0) return;
   EventCounters* c = ws.ev + e;
   uint32_t cum = 0;
   if (c->nHits == 0) {
@@ -389,24 +400,22 @@ __global__ void __launch_bounds__(256, 5) kDoubletWrite(Workspace ws) {
   }
 }
 
-__global__ void kCellsTotal(Workspace ws, uint32_t nEvents) {
-  uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nEvents) return;
+// The doublet totals; clears the per-cell counters of the kernels to come (CA
+// links, tracks).
+__global__ void kCellArrays(Workspace ws) {
+  const uint32_t e = blockIdx.y;
   EventCounters* c = ws.ev + e;
-  uint32_t raw = ws.jOffset[size_t(e) * (ws.cap.jCap + 1) + c->ntot];
+  const uint32_t raw = ws.jOffset[size_t(e) * (ws.cap.jCap + 1) + c->ntot], n = min(raw, ws.cap.cells);
+  uint32_t* nbr = ws.nbrCount + size_t(e) * (ws.cap.cells + 1);
+  uint32_t* trk = ws.trkCount + size_t(e) * (ws.cap.cells + 1);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
+    nbr[i] = 0;
+    trk[i] = 0;
+  }
+  if (blockIdx.x != 0 || threadIdx.x != 0) return;
   c->nCellsRaw = raw;
-  c->nCells = min(raw, ws.cap.cells);
+  c->nCells = n;
   if (raw >= ws.cap.cells) c->flags |= kFlagCellOverflow;
-}
-
-// generic CSR helpers ------------------------------------------------------
-
-// zero n entries of each event's array
-__global__ void kZero(uint32_t* p, size_t stride, uint32_t n, const uint32_t* lenPtr, uint32_t lenStride) {
-  uint32_t e = blockIdx.y;
-  uint32_t len = lenPtr ? min(n, lenPtr[size_t(e) * lenStride] + 1) : n;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x)
-    p[size_t(e) * stride + i] = 0;
 }
 
 // isOuterHitOfCell fill (unordered; lists longer than 128 are ordered after)
@@ -1040,6 +1049,10 @@ __global__ void kNtupletCount(Workspace ws) {
   }
 }
 
+// The tuples to their serial positions, and all that goes with one: its hits'
+// detector indices (kernel_fillHitDetIndices), its share of its cells' track
+// counts, and bulkFinalizeFill with the stored-tuple count (the bins past the
+// last tuple).
 __global__ void kNtupletWrite(Workspace ws) {
   uint32_t e = blockIdx.y;
   EventCounters* c = ws.ev + e;
@@ -1050,79 +1063,83 @@ __global__ void kNtupletWrite(Workspace ws) {
   const uint32_t* ho = ws.startHitOff + size_t(e) * (ws.cap.cells + 1);
   uint32_t* toff = ws.tupleOff + size_t(e) * (ws.cap.tuples + 1);
   uint32_t* th = ws.tupleHits + size_t(e) * ws.cap.tupleHits();
+  uint16_t* td = ws.tupleDet + size_t(e) * ws.cap.tupleHits();
   uint32_t* tcell = ws.tupleCells + size_t(e) * ws.cap.tupleCells();
+  uint32_t* trkCnt = ws.trkCount + size_t(e) * (ws.cap.cells + 1);
   uint8_t* q = ws.quality + size_t(e) * ws.cap.tuples;
+  const uint16_t* det = ws.detInd + size_t(e) * ws.cap.hits;
+  const uint32_t bins = ws.cap.tuples, all = c->apcM;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nThreads = gridDim.x * blockDim.x;
+  for (uint32_t i = all + tid; i <= bins; i += nThreads) toff[i] = c->apcN;
+  if (tid == 0) {
+    if (all >= bins) atomicOr(&c->flags, kFlagTupleOverflow);
+    c->nTuples = min(all, bins);
+  }
+  auto putHit = [&](uint32_t at, uint32_t hit) {
+    th[at] = hit;
+    td[at] = det[hit];
+  };
+  // tuple m starts at off; in a full container the last bin ends where it starts
+  auto putStart = [&](uint32_t m, uint32_t off) {
+    toff[m] = off;
+    if (m == bins - 1 && all >= bins) toff[bins] = off;
+    q[m] = kBad;
+  };
   const TupleStage st = tupleStage(ws, e);
   const uint32_t staged = c->nStaged;
   if (staged <= st.cap) {
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < staged; s += gridDim.x * blockDim.x) {
+    for (uint32_t s = tid; s < staged; s += nThreads) {
       const uint4 r = st.cells[s];
       const uint32_t li = st.start[s];
       const uint32_t m = to[li] + st.rank[s];
-      if (m >= ws.cap.tuples) continue;
+      if (m >= bins) continue;
       const uint32_t off = ho[li] + st.hit[s];
-      toff[m] = off;
+      putStart(m, off);
       // the cells (at least two) and their hits; the per-event stride of
       // tcell is 4 * cap.tuples words on a 256-byte aligned base
-      th[off] = ws.cellInner[cb + r.x];
-      th[off + 1] = ws.cellInner[cb + r.y];
+      putHit(off, ws.cellInner[cb + r.x]);
+      putHit(off + 1, ws.cellInner[cb + r.y]);
+      atomicAdd(&trkCnt[r.x], 1u);
+      atomicAdd(&trkCnt[r.y], 1u);
       uint32_t last = r.y, nc = 2;
       if (r.z != ~0u) {
-        th[off + 2] = ws.cellInner[cb + r.z];
+        putHit(off + 2, ws.cellInner[cb + r.z]);
+        atomicAdd(&trkCnt[r.z], 1u);
         last = r.z;
         nc = 3;
         if (r.w != ~0u) {
-          th[off + 3] = ws.cellInner[cb + r.w];
+          putHit(off + 3, ws.cellInner[cb + r.w]);
+          atomicAdd(&trkCnt[r.w], 1u);
           last = r.w;
           nc = 4;
         }
       }
-      th[off + nc] = ws.cellOuter[cb + last];
+      putHit(off + nc, ws.cellOuter[cb + last]);
       reinterpret_cast<uint4*>(tcell)[m] = r;
-      q[m] = kBad;
     }
     return;
   }
   const uint32_t* linked = ws.candidates + size_t(e) * ws.cap.cells;
-  for (uint32_t li = blockIdx.x * blockDim.x + threadIdx.x; li < c->nLinked; li += gridDim.x * blockDim.x) {
+  for (uint32_t li = tid; li < c->nLinked; li += nThreads) {
     const uint32_t idx = linked[li];
     if (!isStartCell(ws, cb, idx)) continue;
     uint32_t m = to[li], off = ho[li];
-    if (m >= ws.cap.tuples) continue;
+    if (m >= bins) continue;
     dfsNtuplets(idx, ws.cellDoubletId + cb, nbrOff, nbr, ws.ca.minHits, [&](int ncells, const uint32_t* cells) {
-      if (m < ws.cap.tuples) {
-        toff[m] = off;
+      if (m < bins) {
+        putStart(m, off);
         for (int k = 0; k < ncells; ++k) {
-          th[off + k] = ws.cellInner[cb + cells[k]];
+          putHit(off + k, ws.cellInner[cb + cells[k]]);
           tcell[4 * m + k] = cells[k];
+          atomicAdd(&trkCnt[cells[k]], 1u);
         }
-        th[off + ncells] = ws.cellOuter[cb + cells[ncells - 1]];
+        putHit(off + ncells, ws.cellOuter[cb + cells[ncells - 1]]);
         for (int k = ncells; k < 4; ++k) tcell[4 * m + k] = 0xffffffffu;
-        q[m] = kBad;
       }
       ++m;
       off += uint32_t(ncells) + 1;
     });
   }
-}
-
-// bulkFinalizeFill and the stored-tuple count
-__global__ void kTupleFinalize(Workspace ws) {
-  uint32_t e = blockIdx.y;
-  EventCounters* c = ws.ev + e;
-  uint32_t m = c->apcM, nh = c->apcN;
-  uint32_t* toff = ws.tupleOff + size_t(e) * (ws.cap.tuples + 1);
-  const uint32_t bins = ws.cap.tuples;
-  if (m >= bins) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      toff[bins] = toff[bins - 1];
-      c->flags |= kFlagTupleOverflow;
-    }
-  } else {
-    for (uint32_t i = m + blockIdx.x * blockDim.x + threadIdx.x; i <= bins; i += gridDim.x * blockDim.x)
-      toff[i] = nh;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) c->nTuples = min(m, bins);
 }
 
 __device__ __forceinline__ uint32_t tupleSize(const uint32_t* toff, uint32_t t) { return toff[t + 1] - toff[t]; }
@@ -1142,19 +1159,7 @@ __device__ __forceinline__ uint4 tupleCellSlots(const uint32_t* tcell, uint32_t 
   return *reinterpret_cast<const uint4*>(tcell + 4 * size_t(t));
 }
 
-// cell -> track lists: count, (scan), fill, order
-__global__ void kTrackCount(Workspace ws) {
-  uint32_t e = blockIdx.y;
-  EventCounters* c = ws.ev + e;
-  uint32_t nt = c->nTuples;
-  const uint32_t* tcell = ws.tupleCells + size_t(e) * ws.cap.tupleCells();
-  uint32_t* cnt = ws.trkCount + size_t(e) * (ws.cap.cells + 1);
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
-    const uint32_t ncell = tupleCellCount(tcell, t);
-    for (uint32_t k = 0; k < ncell; ++k) atomicAdd(&cnt[tcell[4 * t + k]], 1u);
-  }
-}
-
+// cell -> track lists: counted by kNtupletWrite, (scan), fill, order
 __global__ void kTrackFill(Workspace ws) {
   uint32_t e = blockIdx.y;
   EventCounters* c = ws.ev + e;
@@ -1224,17 +1229,6 @@ __global__ void kEarlyDup(Workspace ws) {
     for (uint32_t j = 0; j < s; ++j)
       if (tupleSize(toff, trk[b + j]) != maxNh) q[trk[b + j]] = kDup;
   }
-}
-
-// tuple hits -> detector indices (kernel_fillHitDetIndices)
-__global__ void kTupleDet(Workspace ws) {
-  uint32_t e = blockIdx.y;
-  const uint32_t* toff = ws.tupleOff + size_t(e) * (ws.cap.tuples + 1);
-  uint32_t n = toff[ws.cap.tuples];
-  const uint32_t* th = ws.tupleHits + size_t(e) * ws.cap.tupleHits();
-  uint16_t* td = ws.tupleDet + size_t(e) * ws.cap.tupleHits();
-  const uint16_t* det = ws.detInd + size_t(e) * ws.cap.hits;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) td[k] = det[th[k]];
 }
 
 // TupleMultiplicity: counts per hit multiplicity, then fill (order irrelevant to the fits)
@@ -1672,21 +1666,17 @@ cudaError_t runCA(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStrea
   const uint32_t gx = nEvents >= 32 ? 16 : (nEvents >= 8 ? 64 : 296);  // blocks per event for flat loops
   dim3 g(gx, nEvents);
   // ---- doublets: count per inner-hit slot, scan, write in serial order
-  PG_PROBED("kDoubletSetup", stream, kDoubletSetup<<<(nEvents + 63) / 64, 64, 0, stream>>>(ws, nEvents));
-  PG_PROBED("kZero", stream, kZero<<<dim3(48, nEvents), 256, 0, stream>>>(ws.ohCount, kHitCap + 1, kHitCap + 1, EVF(nHits)));
+  PG_PROBED("kHitArrays", stream, kHitArrays<<<dim3(48, nEvents), 256, 0, stream>>>(ws));
   PG_PROBED("kDoubletCount", stream, kDoubletCount<<<dim3(tunedGrid(ws, kTuneDoubletCount, gx * 4), nEvents), 256, 0, stream>>>(ws));
   segScan(ws, kScanDoubletSlots, ws.jCount, ws.jOffset, kJCap + 1, EVF(ntot), kJCap, nullptr, 0, nEvents, stream);
   PG_PROBED("kDoubletWrite", stream, kDoubletWrite<<<dim3(tunedGrid(ws, kTuneDoubletWrite, gx * 4), nEvents), 256, 0, stream>>>(ws));
-  PG_PROBED("kCellsTotal", stream, kCellsTotal<<<(nEvents + 63) / 64, 64, 0, stream>>>(ws, nEvents));
+  PG_PROBED("kCellArrays", stream, kCellArrays<<<dim3(gx * 2, nEvents), 256, 0, stream>>>(ws));
   // ---- isOuterHitOfCell: scan of the per-hit counts, unordered fill, order per hit
   segScan(ws, kScanOuterHits, ws.ohCount, ws.ohOff, kHitCap + 1, EVF(nHits), kHitCap, nullptr, 0, nEvents, stream, true);
   PG_PROBED("kOuterHitFill", stream, kOuterHitFill<<<dim3(tunedGrid(ws, kTuneOuterHitFill, gx), nEvents), 256, 0, stream>>>(ws));
   sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.ohCells, kCellCap, ws.ohOff, kHitCap + 1, EVF(nHits), 0, false, kCellCap, 0);
   PG_PROBED("kOhRec", stream, kOhRec<<<dim3(tunedGrid(ws, kTuneOhRec, gx), nEvents), 256, 0, stream>>>(ws));
   // ---- CA links: edges appended unordered, then CSR by inner cell, ordered ascending
-  PG_PROBED("kZero", stream, kZero<<<dim3(gx * 2, nEvents), 256, 0, stream>>>(ws.nbrCount, kCellCap + 1, kCellCap + 1, EVF(nCells)));
-  if (ws.ca.earlyFishbone)
-    PG_PROBED("kZero", stream, kZero<<<dim3(gx, nEvents), 256, 0, stream>>>(ws.hitTouch, kHitCap, kHitCap, EVF(nHits)));
   PG_PROBED("kConnect", stream, kConnect<<<dim3(tunedGrid(ws, kTuneConnect, gx * 4), nEvents), kConnectWarps * 32, 0, stream>>>(ws, ws.scratchA, ws.scratchB));
   // (the linked cells' list stays in ws.candidates until kTrackPool)
   segScanList(ws, kScanNeighbours, ws.nbrCount, ws.nbrOff, kScanLinked, ws.candidates, &ws.ev[0].nLinked, kCellCap + 1,
@@ -1703,10 +1693,7 @@ cudaError_t runCA(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStrea
            ws.startHitOff, &ws.ev[0].apcN, kCellCap + 1, EVF(nLinked), kCellCap, sizeof(EventCounters) / 4, nEvents,
            stream);
   PG_PROBED("kNtupletWrite", stream, kNtupletWrite<<<dim3(tunedGrid(ws, kTuneNtupletWrite, gx * 8), nEvents), 128, 0, stream>>>(ws));
-  PG_PROBED("kTupleFinalize", stream, kTupleFinalize<<<dim3(32, nEvents), 1024, 0, stream>>>(ws));
   // ---- cell -> track lists
-  PG_PROBED("kZero", stream, kZero<<<dim3(gx * 2, nEvents), 256, 0, stream>>>(ws.trkCount, kCellCap + 1, kCellCap + 1, EVF(nCells)));
-  PG_PROBED("kTrackCount", stream, kTrackCount<<<dim3(tunedGrid(ws, kTuneTrackCount, gx), nEvents), 256, 0, stream>>>(ws));
   segScan(ws, kScanCellTracks, ws.trkCount, ws.trkOff, kCellCap + 1, EVF(nCells), kCellCap, nullptr, 0, nEvents, stream,
           true);
   PG_PROBED("kTrackFill", stream, kTrackFill<<<dim3(tunedGrid(ws, kTuneTrackFill, gx), nEvents), 256, 0, stream>>>(ws));
@@ -1714,7 +1701,6 @@ cudaError_t runCA(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStrea
   uint32_t* candFlag = ws.startTupleCount;  // scratch
   PG_PROBED("kTrackPool", stream, kTrackPool<<<dim3(tunedGrid(ws, kTuneTrackPool, gx), nEvents), 256, 0, stream>>>(ws, candFlag));
   PG_PROBED("kEarlyDup", stream, kEarlyDup<<<dim3(tunedGrid(ws, kTuneEarlyDup, gx), nEvents), 256, 0, stream>>>(ws));
-  PG_PROBED("kTupleDet", stream, kTupleDet<<<dim3(tunedGrid(ws, kTuneTupleDet, gx), nEvents), 256, 0, stream>>>(ws));
   // ---- tuple multiplicity for the fits
   cudaError_t le = cudaSuccess;
   PG_PROBED("kMultiplicity", stream,
@@ -1745,7 +1731,6 @@ cudaError_t runCleaners(Workspace& ws, uint32_t nEvents, cudaStream_t stream) {
             le = launchClustered(kFastDupRounds, P, nEvents, kFastDupThreads, 0, stream, ws, indeg, lists, candFlag));
   if (le != cudaSuccess) return le;
   // hit -> tuple map and triplet cleaner
-  PG_PROBED("kZero", stream, kZero<<<dim3(48, nEvents), 256, 0, stream>>>(ws.h2tCount, kHitCap + 1, kHitCap + 1, EVF(nHits)));
   PG_PROBED("kHitToTupleCount", stream, kHitToTupleCount<<<dim3(tunedGrid(ws, kTuneHitToTupleCount, gx), nEvents), 256, 0, stream>>>(ws));
   segScan(ws, kScanHitTuples, ws.h2tCount, ws.h2tOff, kHitCap + 1, EVF(nHits), kHitCap, nullptr, 0, nEvents, stream, true);
   PG_PROBED("kHitToTupleFill", stream, kHitToTupleFill<<<dim3(tunedGrid(ws, kTuneHitToTupleFill, gx), nEvents), 256, 0, stream>>>(ws));

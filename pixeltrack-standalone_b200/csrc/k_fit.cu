@@ -685,8 +685,11 @@ cudaError_t runFits(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStr
   // one wave of blocks of 512 threads per SM; a few events' tuples (a PU50 event
   // has 10.6k) go in tiles of 64, over all SMs.  The launch table does not scale
   // this grid: it follows from the SMs alone.
+  // Otherwise tiles of 128: the hits' gathers make the block wait, and two more
+  // blocks per SM fill that better than one wide block in step (64 PU50 events:
+  // 174 us with 256, 167 us with 128).
   const uint32_t most = riemann ? kRiemannBlock : kFitBlock;
-  const uint32_t fb = nEvents <= 4 ? 64u : most, fg = 148 * (512 / fb);
+  const uint32_t fb = nEvents <= 4 ? 64u : 128u, fg = 148 * (512 / fb);
   static std::atomic<uint64_t> configured[4];
   cudaError_t le = cudaSuccess;
   auto launch = [&](int which, auto kernel) {

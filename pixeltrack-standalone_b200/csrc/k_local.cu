@@ -180,7 +180,6 @@ __global__ void kInitEvents(Workspace ws, uint32_t nEvents) {
     c->apcM = c->apcN = c->nTuples = c->nTupleCells = 0;
     c->nCandidates = c->nLoose = 0;
     c->nVertices = c->nErrors = c->nVtxTracks = 0;
-    c->nBig[0] = c->nBig[1] = c->nBig[2] = c->nBig[3] = 0;
     c->nBigMod = 0;
     c->nSegList[0] = c->nSegList[1] = c->nSegList[2] = c->nSegList[3] = 0;
     c->nBigHitMod = 0;
@@ -883,10 +882,15 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 7) kFindClustersSmall(Worksp
   }
 }
 
-// fillHitsModuleStart + setHitsLayerStart + beam-spot corrected average geometry
-__global__ void kHitsModuleStart(DeviceES es, Workspace ws) {
+// fillHitsModuleStart + setHitsLayerStart + beam-spot corrected average geometry;
+// clears the phi histogram's counters and fill cursors for the kernels that follow
+__global__ void kHitsModuleStart(DeviceES es, Workspace ws, uint32_t* phiCursor) {
   __shared__ uint32_t scanSh[33];
   uint32_t e = blockIdx.x;
+  for (uint32_t i = threadIdx.x; i < kPhiStride; i += blockDim.x) {
+    ws.phiOff[size_t(e) * kPhiStride + i] = 0;
+    phiCursor[size_t(e) * kPhiStride + i] = 0;
+  }
   const uint32_t* cim = ws.clusInModule + size_t(e) * kModStride;
   uint32_t* cms = ws.clusModuleStart + size_t(e) * kModStride;
   uint32_t carry = 0;
@@ -1222,12 +1226,6 @@ __global__ void kPhiRec(Workspace ws) {
   }
 }
 
-__global__ void kZeroU32(uint32_t* p, size_t stride, uint32_t n, uint32_t nEvents) {
-  uint32_t e = blockIdx.y;
-  if (e >= nEvents) return;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[e * stride + i] = 0;
-}
-
 // order each event's error list by word index (the serial push order)
 __global__ void kSortErrors(Workspace ws) {
   uint32_t e = blockIdx.x;
@@ -1278,15 +1276,13 @@ cudaError_t runLocal(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaSt
             kFindClustersSmall<<<dim3((kMaxModules + kSmallWarps - 1) / kSmallWarps, nEvents), kSmallWarps * 32, 0,
                                  stream>>>(ws));
   PG_PROBED("kFindClustersBig", stream, kFindClustersBig<<<dim3(tunedGrid(ws, kTuneFindClustersBig, 64), nEvents), kClusThreads, 0, stream>>>(ws));
-  PG_PROBED("kHitsModuleStart", stream, kHitsModuleStart<<<nEvents, 1024, 0, stream>>>(es, ws));
+  uint32_t* cursor = ws.jCount;  // scratch: the doublet counters are not in use yet
+  PG_PROBED("kHitsModuleStart", stream, kHitsModuleStart<<<nEvents, 1024, 0, stream>>>(es, ws, cursor));
   PG_PROBED("kGetHits", stream,
             kGetHitsSmall<<<dim3((kMaxModules + kHitWarps - 1) / kHitWarps, nEvents), kHitWarps * 32, 0, stream>>>(es,
                                                                                                                ws));
   PG_PROBED("kGetHitsBig", stream, kGetHitsBig<<<dim3(tunedGrid(ws, kTuneGetHitsBig, 64), nEvents), kHitThreads, 0, stream>>>(es, ws));
   // phi histogram: count, exclusive scan, unordered fill, per-bin ordering
-  uint32_t* cursor = ws.jCount;  // scratch: the doublet counters are not in use yet
-  PG_PROBED("kZeroU32", stream, kZeroU32<<<dim3(2, nEvents), 1024, 0, stream>>>(ws.phiOff, kPhiStride, kPhiStride, nEvents));
-  PG_PROBED("kZeroU32", stream, kZeroU32<<<dim3(2, nEvents), 1024, 0, stream>>>(cursor, kPhiStride, kPhiStride, nEvents));
   PG_PROBED("kPhiCount", stream, kPhiCount<<<dim3(tunedGrid(ws, kTunePhiCount, 16), nEvents), 256, 0, stream>>>(ws));
   // in place exclusive scan of the 1280 counters; the total lands in the extra bin
   segScan(ws, kScanPhi, ws.phiOff, ws.phiOff, kPhiStride, nullptr, 0, kPhiTot - 1, nullptr, 0, nEvents, stream);

@@ -8,8 +8,7 @@
 //              a second entry): n <= 32 sorted in registers by a bitonic
 //              network; 32 < n <= 256 handed to the warp (rank sort, one
 //              segment at a time, ballot over the lanes that hold one);
-//              n > 256 appended to a per-event list for kSortBig.
-//  kSortBig    one block per long segment: rank sort in shared memory.
+//              n > 256 by the whole block, a rank sort in shared memory.
 #pragma once
 
 #include "device_utils.cuh"
@@ -63,9 +62,11 @@ __device__ void serialSort(T* seg, uint32_t n, bool desc) {
 }
 
 template <typename T>
-__global__ void kSortListed(T* data, size_t dataStride, const uint32_t* off, size_t offStride, const uint32_t* list,
-                            size_t listStride, const uint32_t* nList, uint32_t nListStride, bool desc,
-                            uint32_t dataCap, uint32_t* big, uint32_t* nBig, uint32_t nBigStride) {
+__global__ void __launch_bounds__(256) kSortListed(T* data, size_t dataStride, const uint32_t* off, size_t offStride,
+                                                   const uint32_t* list, size_t listStride, const uint32_t* nList,
+                                                   uint32_t nListStride, bool desc, uint32_t dataCap) {
+  __shared__ T sh[kBigSort];
+  __shared__ uint32_t sLong[256], sNLong;
   const uint32_t e = blockIdx.y;
   const uint32_t nseg = nList[size_t(e) * nListStride];
   const uint32_t* o = off + size_t(e) * offStride;
@@ -90,52 +91,38 @@ __global__ void kSortListed(T* data, size_t dataStride, const uint32_t* off, siz
       const uint32_t bb = __shfl_sync(0xffffffffu, b, l), nn = __shfl_sync(0xffffffffu, n, l);
       warpSortSegment(d + bb, nn, desc);
     }
-    if (n > 256) {
-      const uint32_t q = atomicAdd(&nBig[size_t(e) * nBigStride], 1u);
-      if (q < kBigSegCap)
-        big[size_t(e) * kBigSegCap + q] = s;
-      else
-        serialSort(d + b, n, desc);  // more long segments than the list holds
-    }
-  }
-}
-
-template <typename T>
-__global__ void kSortBig(T* data, size_t dataStride, const uint32_t* off, size_t offStride, bool desc,
-                         uint32_t dataCap, const uint32_t* big, const uint32_t* nBig, uint32_t nBigStride) {
-  __shared__ T sh[kBigSort];
-  const uint32_t e = blockIdx.y;
-  const uint32_t nb = min(nBig[size_t(e) * nBigStride], kBigSegCap);
-  const uint32_t* o = off + size_t(e) * offStride;
-  T* d = data + size_t(e) * dataStride;
-  for (uint32_t k = blockIdx.x; k < nb; k += gridDim.x) {
-    const uint32_t s = big[size_t(e) * kBigSegCap + k];
-    const uint32_t b = min(o[s], dataCap), n = min(o[s + 1], dataCap) - b;
-    if (n <= kBigSort) {
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sh[i] = d[b + i];
-      __syncthreads();
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const T v = sh[i];
-        uint32_t r = 0;
-        for (uint32_t j = 0; j < n; ++j) r += desc ? (sh[j] > v) : (sh[j] < v);
-        d[b + r] = v;
-      }
-    } else if (threadIdx.x == 0) {
-      serialSort(d + b, n, desc);
-    }
+    // long segments (none in most events): the block takes them in turn
+    if (!__syncthreads_or(n > 256)) continue;
+    if (threadIdx.x == 0) sNLong = 0;
     __syncthreads();
+    if (n > 256) sLong[atomicAdd(&sNLong, 1u)] = s;
+    __syncthreads();
+    for (uint32_t q = 0; q < sNLong; ++q) {
+      const uint32_t bb = min(o[sLong[q]], dataCap), nn = min(o[sLong[q] + 1], dataCap) - bb;
+      if (nn <= kBigSort) {
+        for (uint32_t i = threadIdx.x; i < nn; i += blockDim.x) sh[i] = d[bb + i];
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < nn; i += blockDim.x) {
+          const T v = sh[i];
+          uint32_t r = 0;
+          for (uint32_t j = 0; j < nn; ++j) r += desc ? (sh[j] > v) : (sh[j] < v);
+          d[bb + r] = v;
+        }
+      } else if (threadIdx.x == 0) {
+        serialSort(d + bb, nn, desc);
+      }
+      __syncthreads();
+    }
   }
 }
 
 // Orders segment s = [off[s], off[s+1]) of data for every segment the
-// preceding fill noted in list `slot` (those with >= 2 entries); `slot` also
-// picks the per-event long-segment counter.  lenPtr/fixedLen (the number of
+// preceding fill noted in list `slot` (those with >= 2 entries).  lenPtr/fixedLen (the number of
 // segments) are kept for the callers' readability only.
 template <typename T>
 void sortSegments(Workspace& ws, uint32_t nEvents, cudaStream_t stream, uint32_t gx, T* data, size_t dataStride,
                   const uint32_t* off, size_t offStride, const uint32_t* lenPtr, uint32_t lenStride, uint32_t fixedLen,
                   bool desc, uint32_t dataCap, int slot) {
-  uint32_t* nBig = &ws.ev[0].nBig[slot];
   const uint32_t stride = sizeof(EventCounters) / 4;
   (void)lenPtr;
   (void)lenStride;
@@ -143,10 +130,7 @@ void sortSegments(Workspace& ws, uint32_t nEvents, cudaStream_t stream, uint32_t
   PG_PROBED("kSortSegments", stream,
             kSortListed<T><<<dim3(gx, nEvents), 256, 0, stream>>>(data, dataStride, off, offStride, ws.segList,
                                                                   ws.cap.cells, &ws.ev[0].nSegList[slot], stride,
-                                                                  desc, dataCap, ws.bigSeg, nBig, stride));
-  PG_PROBED("kSortBig", stream,
-            kSortBig<T><<<dim3(8, nEvents), 256, 0, stream>>>(data, dataStride, off, offStride, desc, dataCap,
-                                                              ws.bigSeg, nBig, stride));
+                                                                  desc, dataCap));
 }
 
 }  // namespace pixgpu

@@ -192,7 +192,8 @@ int pg_autotune(pg_ctx* c, uint32_t n, const uint8_t* const* raws, const size_t*
   };
   for (uint32_t id = 0; id < kNumTune && rc == PG_OK; ++id) {
     if (id == kTuneFedCopy && !c->cfg.fed_scan) continue;
-    if (id == kTuneNbrPool) continue;  // no longer launched; saved tables name it
+    // names that saved tables hold, of work that other kernels do now
+    if (id == kTuneNbrPool || id == kTuneTrackCount || id == kTuneTupleDet || id == kTuneFit) continue;
     if ((rc = pg_set_probe(c, launchedName(c, id))) != PG_OK) break;
     const int start = tuningFor(c, n).scale[id];
     double best = 0;
