@@ -138,14 +138,18 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
     fc2 = f2;
     ff[3] = float(f2 * atan2(cross2D(dx, dy, ex, ey), dx * ex + dy * ey) / (Hd(2, n - 1) - Hd(2, 0)));
   }
+  PG_FIT_PHASE();
+  // formed once, as in blFit: the slope and its rotation, the scattering
+  // variance of the first step, the hits' radii
   int q;
-  float radii[2][N], s[N], S[N], Z[N], VarBeta[N];
+  float radii[2][N], radf[N], s[N], S[N], Z[N], VarBeta[N], slope, ms01;
+  MF<2, 2> R;
   {
     float dx = H(0, 1) - H(0, 0), dy = H(1, 1) - H(1, 0);
     float ex = H(0, n - 1) - H(0, n - 2), ey = H(1, n - 1) - H(1, n - 2);
     q = cross2DF(dx, dy, ex, ey) > 0 ? -1 : 1;
-    const float slope = -q / ff[3];
-    MF<2, 2> R = rotationMatrixF(slope);
+    slope = -q / ff[3];
+    R = rotationMatrixF(slope);
     // the arc lengths in FP64: the radius vectors are as long as the radius
     // (metres for a stiff track) and the angles between them small, so in
     // FP32 their cross products, and the circle centre itself, would carry
@@ -157,6 +161,7 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
       rd[1][i] = double(H(1, i)) - fc1;
       radii[0][i] = float(rd[0][i]);
       radii[1][i] = float(rd[1][i]);
+      radf[i] = sqrtf(radii[0][i] * radii[0][i] + radii[1][i] * radii[1][i]);
     }
     // the circle centre in the beam-line frame gives the direction of the
     // point of closest approach
@@ -172,18 +177,22 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
       S[i] = R(0, 0) * p0 + R(0, 1) * p1;
       Z[i] = R(1, 0) * p0 + R(1, 1) * p1;
     }
+    PG_FIT_PHASE();
     VarBeta[0] = VarBeta[n - 1] = 0;
+    float ms = ms01 = multScattF(S[1] - S[0], Bf, ff[2], slope);
 #pragma unroll
-    for (int i = 1; i < n - 1; ++i)
-      VarBeta[i] = multScattF(S[i + 1] - S[i], Bf, ff[2], slope) + multScattF(S[i] - S[i - 1], Bf, ff[2], slope);
+    for (int i = 1; i < n - 1; ++i) {
+      const float next = multScattF(S[i + 1] - S[i], Bf, ff[2], slope);
+      VarBeta[i] = next + ms;
+      ms = next;
+    }
   }
+  PG_FIT_PHASE();
   // ---- line fit
   float lpar[2];
   M<2, 2> lcov;
   float lchi2;
   {
-    const float slope = -q / ff[3];
-    MF<2, 2> R = rotationMatrixF(slope);
     MF<3, 3> V;
     MF<2, 3> J;
 #pragma unroll
@@ -200,13 +209,14 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
       V(1, 1) = g[2];
       V(2, 1) = V(1, 2) = g[4];
       V(2, 2) = g[5];
-      float tmp = 1.f / sqrtf(radii[0][i] * radii[0][i] + radii[1][i] * radii[1][i]);
+      float tmp = 1.f / radf[i];
       J(0, 0) = radii[1][i] * tmp;
       J(0, 1) = -radii[0][i] * tmp;
       J(1, 2) = 1.f;
       MF<2, 2> P = mulf(mulf(mulf(mulf(R, J), V), trf(J)), trf(R));
       w[i] = 1.f / P(1, 1);
     }
+    PG_FIT_PHASE();
     M<N, N> I;
     invertToDouble<N>(matrixCuF<N>(w, S, VarBeta), I);
     double u[N];
@@ -220,7 +230,7 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
     lpar[0] = float(u[1] - u[0]) / (S[1] - S[0]);
     lpar[1] = float(u[0]);
     const double idiff = 1. / double(S[1] - S[0]);
-    lcov(0, 0) = (I(0, 0) - 2 * I(0, 1) + I(1, 1)) * sqr(idiff) + double(multScattF(S[1] - S[0], Bf, ff[2], slope));
+    lcov(0, 0) = (I(0, 0) - 2 * I(0, 1) + I(1, 1)) * sqr(idiff) + double(ms01);
     lcov(0, 1) = (I(0, 1) - I(0, 0)) * idiff;
     lcov(1, 0) = (I(0, 1) - I(0, 0)) * idiff;
     lcov(1, 1) = I(0, 0);
@@ -251,12 +261,12 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
                  VarBeta[i];
     }
   }
+  PG_FIT_PHASE();
   // ---- circle fit
   double cpar[3];
   M<3, 3> ccov;
   float cchi2;
   {
-    const float slope = -q / ff[3];
 #pragma unroll
     for (int i = 0; i < n; ++i) VarBeta[i] *= 1.f + sqrf(slope);
 #pragma unroll
@@ -278,6 +288,7 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
       MF<2, 2> P = mulf(mulf(RR, V), trf(RR));
       w[i] = 1.f / P(1, 1);
     }
+    PG_FIT_PHASE();
     MF<N + 1, N + 1> C;
     {
       MF<N, N> cu = matrixCuF<N>(w, s, VarBeta);
@@ -298,6 +309,7 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
       C(n, i) = C(i, n);
       if (i > 0 && i < n - 1) C(n, n) += sqrf(s[i + 1] - s[i - 1]) / (4.f * VarBeta[i]);
     }
+    PG_FIT_PHASE();
     M<N + 1, N + 1> I;
     invertToDouble<N + 1>(C, I);
     double u[N + 1];
@@ -310,9 +322,8 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
     }
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      const float nr = sqrtf(radii[0][c] * radii[0][c] + radii[1][c] * radii[1][c]);
-      radii[0][c] /= nr;
-      radii[1][c] /= nr;
+      radii[0][c] /= radf[c];
+      radii[1][c] /= radf[c];
     }
     const float u0 = float(u[0]), u1 = float(u[1]);
     const float dx = H(0, 0) + (-Z[0] + u0) * radii[0][0], dy = H(1, 0) + (-Z[0] + u0) * radii[1][0];
@@ -324,28 +335,20 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
     cpar[1] = double(-q * (quarter / (ff[2] + sqrtf(sqrf(ff[2]) - quarter))));
     cpar[2] = double(q * (1.f / ff[2] + float(u[n])));
     const float tmp1 = emdx * emdx + emdy * emdy;
-    M<3, 3> J;
-    J(0, 0) = double((radii[1][0] * emdx - emdy * radii[0][0]) / tmp1);
-    J(0, 1) = double((radii[1][1] * emdx - emdy * radii[0][1]) / tmp1);
-    J(0, 2) = 0;
-    J(1, 0) = double((q / 2) * (emdx * radii[0][0] + emdy * radii[1][0]) / sqrtf(sqrf(2 * ff[2]) - tmp1));
-    J(1, 1) = double((q / 2) * (emdx * radii[0][1] + emdy * radii[1][1]) / sqrtf(sqrf(2 * ff[2]) - tmp1));
-    J(1, 2) = 0;
-    J(2, 0) = 0;
-    J(2, 1) = 0;
-    J(2, 2) = q;
-    ccov(0, 0) = I(0, 0);
-    ccov(0, 1) = I(0, 1);
-    ccov(0, 2) = I(0, n);
-    ccov(1, 0) = I(1, 0);
-    ccov(1, 1) = I(1, 1);
-    ccov(1, 2) = I(1, n);
-    ccov(2, 0) = I(n, 0);
-    ccov(2, 1) = I(n, 1);
-    ccov(2, 2) = I(n, n);
-    ccov = sandwich(J, ccov);
-    translateKarimaki<false>(cpar, ccov, 0.5 * double(emdx), 0.5 * double(emdy));
-    ccov(0, 0) += double((1.f + sqrf(slope)) * multScattF(S[1] - S[0], Bf, ff[2], slope));
+    // the Jacobian of blFit, whose elements of dca are zero
+    const double a0 = double((radii[1][0] * emdx - emdy * radii[0][0]) / tmp1);
+    const double a1 = double((radii[1][1] * emdx - emdy * radii[0][1]) / tmp1);
+    const double t00 = a0 * I(0, 0) + a1 * I(1, 0), t01 = a0 * I(0, 1) + a1 * I(1, 1);
+    const double t02 = a0 * I(0, n) + a1 * I(1, n);
+    const double t20 = q * I(n, 0), t21 = q * I(n, 1), t22 = q * I(n, n);
+    ccov(0, 0) = t00 * a0 + t01 * a1;
+    ccov(0, 2) = t02 * q;
+    ccov(2, 0) = t20 * a0 + t21 * a1;
+    ccov(2, 2) = t22 * q + 0. * (I(0, 0) + I(0, 1) + I(1, 1) + I(0, n) + I(1, n));
+    PG_FIT_PHASE();
+    translateKarimaki<true>(cpar, ccov, 0.5 * double(emdx), 0.5 * double(emdy));
+    ccov(0, 0) += double((1.f + sqrf(slope)) * ms01);
+    PG_FIT_PHASE();
     translateKarimaki<false>(cpar, ccov, double(dx) + x0, double(dy) + y0);
     cchi2 = 0;
 #pragma unroll
