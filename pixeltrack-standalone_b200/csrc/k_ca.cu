@@ -1431,7 +1431,7 @@ __global__ void kFastDupInDegree(Workspace ws, uint32_t* indeg, const uint32_t* 
 }
 
 // One thread-block cluster of P CTAs per event (kFastDupCtas for small
-// batches, 2 for large ones).  A worklist
+// batches, 4 for larger and 2 for large ones).  A worklist
 // holds the candidates whose earlier track-sharing candidates are all done;
 // cells of one round share no track, so the cluster's threads process them in
 // parallel, and each releases its later neighbours (the in-degree reaching
@@ -1725,7 +1725,8 @@ cudaError_t runCleaners(Workspace& ws, uint32_t nEvents, cudaStream_t stream) {
   uint32_t* indeg = ws.scratchA;        // [maxEvents][cap.scratch], cap.cells per event used
   uint32_t* lists = ws.scratchB;        // two worklists of cap.cells per event (cap.scratch >= 2 cap.cells)
   PG_PROBED("kFastDupInDegree", stream, kFastDupInDegree<<<dim3(tunedGrid(ws, kTuneFastDupInDegree, gx), nEvents), 256, 0, stream>>>(ws, indeg, candFlag));
-  const uint32_t P = nEvents <= kClusterMaxEvents ? kFastDupCtas : 2;
+  // 24 dense events: 148 us in pairs, 116 us on four CTAs each; 64 PU50 events: 108 us in pairs, 116 us on four
+  const uint32_t P = nEvents <= kClusterMaxEvents ? kFastDupCtas : (nEvents <= 2 * kClusterMaxEvents ? 4u : 2u);
   cudaError_t le = cudaSuccess;
   PG_PROBED("kFastDupRounds", stream,
             le = launchClustered(kFastDupRounds, P, nEvents, kFastDupThreads, 0, stream, ws, indeg, lists, candFlag));
