@@ -336,7 +336,8 @@ int pg_probe_read(pg_ctx* ctx, uint32_t slot, uint32_t max, pg_probe_entry* out,
  * 2^scale, scale in -3..3 (0: default), kept per batch size (a batch uses the
  * table of its size, else of the largest tuned size below it).  Results do
  * not depend on the scales.  pg_tune_kernel_name(i) names the i-th tunable
- * kernel (NULL past the last).  pg_tune_set/pg_tune_load need every slot free
+ * kernel (NULL past the last); kNbrPool, kTrackCount, kTupleDet and kBLFit are
+ * kept for saved tables and scale nothing.  pg_tune_set/pg_tune_load need every slot free
  * and drop the captured graphs.
  * pg_autotune times each tunable kernel (kernel probe, median of `repeats`
  * batches of the first n records) at scales -2..2 and keeps the fastest when

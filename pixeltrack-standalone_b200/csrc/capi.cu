@@ -333,8 +333,21 @@ int stage(pg_ctx* c, Slot& s, uint32_t nEvents, const uint8_t* const* raws, cons
   return PG_OK;
 }
 
+// The slot's side stream, made when its first batch is launched or captured (by
+// the thread that holds the slot, outside any capture): a context that only
+// fits tuples or clusters digis has no use for it.
+int ensureSide(pg_ctx* c, Slot& s) {
+  cudaError_t e = cudaSuccess;
+  if (!s.side.fork) e = cudaEventCreateWithFlags(&s.side.fork, cudaEventDisableTiming);
+  if (e == cudaSuccess && !s.side.join) e = cudaEventCreateWithFlags(&s.side.join, cudaEventDisableTiming);
+  if (e == cudaSuccess && !s.side.stream) e = cudaStreamCreateWithFlags(&s.side.stream, cudaStreamNonBlocking);
+  return e == cudaSuccess ? PG_OK : cudaFail(c, e, "side stream");
+}
+
 // Captures runChain + result packing for `n` events on the slot's stream.
 int captureGraph(pg_ctx* c, Slot& s, uint32_t n, cudaGraphExec_t* out) {
+  const int sr = ensureSide(c, s);
+  if (sr != PG_OK) return sr;
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cudaFail(c, e, "begin capture");
@@ -391,6 +404,8 @@ int pixgpu::launchBatch(pg_ctx* c, Slot& s) {
     e = cudaGraphLaunch(s.graphs[s.nEvents], s.stream);
     if (e != cudaSuccess) return cudaFail(c, e, "graph launch");
   } else {
+    const int sr = ensureSide(c, s);
+    if (sr != PG_OK) return sr;
     KernelProbe* pr = c->probeName.empty() ? nullptr : s.probe;
     if (pr) pr->used = 0;
     tProbe = pr;
@@ -463,9 +478,6 @@ int createSlot(pg_ctx* c, Slot& s, size_t bytes) {
   s.ws.ca.lateFishbone = c->cfg.late_fishbone != 0;
   s.ws.ca.mixedFit = c->cfg.mixed_fit != 0;
   if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&s.side.stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&s.side.fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&s.side.join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&s.gathered, cudaEventDisableTiming) != cudaSuccess ||
       cudaMallocHost(&s.hWords, size_t(c->cfg.max_words_per_batch) * 4) != cudaSuccess ||
