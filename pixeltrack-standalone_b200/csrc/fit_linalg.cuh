@@ -31,6 +31,18 @@ struct FitTile {
   static constexpr int kBytes = kHitStride * 8 + kGeStride * 4;  // per tuple; the results take 80
 };
 
+// The places of a thread's inputs in the chain fits' shared memory, in doubles
+// and in floats from its start: the same for 3 and 4 hits, so that no thread
+// ever writes where another one reads, on whichever tiles the two are.
+struct ChainTile {
+  using Widest = FitTile<4>;
+  static constexpr int kBytes = Widest::kBytes;
+  static __device__ __forceinline__ uint32_t hits(uint32_t thread) { return thread * Widest::kHitStride; }
+  static __device__ __forceinline__ uint32_t ge(uint32_t thread, uint32_t threads) {
+    return threads * Widest::kHitStride * 2 + thread * Widest::kGeStride;
+  }
+};
+
 __device__ __forceinline__ double sqr(double a) { return a * a; }
 
 template <int R, int C>

@@ -438,7 +438,7 @@ __device__ __forceinline__ uint32_t fitBinPrefix(const Workspace& ws, uint32_t n
 template <int N, int kMode>
 __device__ __forceinline__ void fitTile(const DeviceES& es, const Workspace& ws, uint32_t nh, uint32_t nEvents,
                                         const uint32_t* pre, uint32_t g0, uint32_t total) {
-  extern __shared__ double tile[];  // the threads' inputs (FitTile)
+  extern __shared__ double tile[];  // the threads' inputs (ChainTile)
   const double B = double(float(0.0114256972711507));
   // the block fits in step (PG_FIT_PHASE): threads past the end repeat the last item
   const bool live = g0 + threadIdx.x < total;
@@ -461,8 +461,11 @@ __device__ __forceinline__ void fitTile(const DeviceES& es, const Workspace& ws,
   const size_t tb = size_t(e) * ws.cap.tuples;
   uint32_t tkid = bins[start + k];
   const uint32_t* hid = th + toff[tkid];
-  double* H = reinterpret_cast<double*>(tile) + threadIdx.x * FitTile<N>::kHitStride;
-  float* ge = reinterpret_cast<float*>(tile + blockDim.x * FitTile<N>::kHitStride) + threadIdx.x * FitTile<N>::kGeStride;
+  // only this thread's, whichever N the block's other warps are at: the Riemann
+  // fits have no barrier, and a warp ahead of the others fills its next tile
+  // while they still read theirs
+  double* H = tile + ChainTile::hits(threadIdx.x);
+  float* ge = reinterpret_cast<float*>(tile) + ChainTile::ge(threadIdx.x, blockDim.x);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     uint32_t hit = hid[i];
@@ -693,7 +696,7 @@ cudaError_t runFits(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStr
   static std::atomic<uint64_t> configured[4];
   cudaError_t le = cudaSuccess;
   auto launch = [&](int which, auto kernel) {
-    le = launchFit(kernel, configured[which], most, fg, fb, FitTile<4>::kBytes, stream, es, ws, nEvents);
+    le = launchFit(kernel, configured[which], most, fg, fb, ChainTile::kBytes, stream, es, ws, nEvents);
   };
   if (riemann && ws.ca.mixedFit)
     PG_PROBED("kRiemannFitMixed", stream, launch(0, kRiemannFitMixed));

@@ -61,3 +61,14 @@ extern "C" int hf_fit_riemann(int N, int mixed, uint32_t n, const double* hits, 
     return -1;
   return 0;
 }
+
+// Byte range [out[0], out[1]) of the hits and [out[2], out[3]) of the covariances
+// of an N-hit tuple that thread `thread` of `threads` holds in the chain fits'
+// shared memory; returns the bytes of the block's shared memory.
+extern "C" uint32_t hf_chain_tile(int N, uint32_t thread, uint32_t threads, uint32_t* out) {
+  out[0] = ChainTile::hits(thread) * 8;
+  out[1] = out[0] + 3 * N * 8;
+  out[2] = ChainTile::ge(thread, threads) * 4;
+  out[3] = out[2] + 6 * N * 4;
+  return threads * ChainTile::kBytes;
+}

@@ -28,6 +28,8 @@ def host_lib():
     lib = ctypes.CDLL(out)
     lib.hf_fit_riemann.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_uint32] + [ctypes.c_void_p] * 2 + \
         [ctypes.c_double] + [ctypes.c_void_p] * 5
+    lib.hf_chain_tile.argtypes = [ctypes.c_int] + [ctypes.c_uint32] * 2 + [ctypes.c_void_p]
+    lib.hf_chain_tile.restype = ctypes.c_uint32
     return lib
 
 
@@ -61,3 +63,21 @@ def test_mixed_riemann_stays_finite_where_single_precision_cancels(host_lib, nh,
     hits, ge, _ = pixgpu.fit_tuples(4242 + nh, index + 1, nh)
     got = host_fit(host_lib, N, hits[index:], ge[index:], True)
     assert np.isfinite(got["state"]).all() and np.isfinite(got["pt"]).all()
+
+
+@pytest.mark.parametrize("threads", [64, 128, 256])
+def test_a_thread_of_the_chain_fits_writes_only_its_own_inputs(host_lib, threads):
+    """The warps of a block may be at different tiles, one at 4-hit tuples
+    while the next is at 3-hit ones: no byte that a thread fills for one width
+    is another thread's for either width, and all lie in the block's memory."""
+    owner = None
+    for N in (3, 4):
+        for t in range(threads):
+            r = (ctypes.c_uint32 * 4)()
+            size = host_lib.hf_chain_tile(N, t, threads, r)
+            if owner is None:
+                owner = np.full(size, -1)
+            for a, b in ((r[0], r[1]), (r[2], r[3])):
+                assert a < b <= size and a % 4 == 0
+                assert np.isin(owner[a:b], (-1, t)).all(), (N, t)
+                owner[a:b] = t
