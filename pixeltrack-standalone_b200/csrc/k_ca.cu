@@ -1070,7 +1070,10 @@ __global__ void kNtupletWrite(Workspace ws) {
   const uint16_t* det = ws.detInd + size_t(e) * ws.cap.hits;
   const uint32_t bins = ws.cap.tuples, all = c->apcM;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nThreads = gridDim.x * blockDim.x;
-  for (uint32_t i = all + tid; i <= bins; i += nThreads) toff[i] = c->apcN;
+  // the empty bins past the last tuple; a full container (exactly as many
+  // tuples as bins included) has none, and its end is putStart's alone
+  if (all < bins)
+    for (uint32_t i = all + tid; i <= bins; i += nThreads) toff[i] = c->apcN;
   if (tid == 0) {
     if (all >= bins) atomicOr(&c->flags, kFlagTupleOverflow);
     c->nTuples = min(all, bins);

@@ -82,3 +82,28 @@ def test_tuple_overflow_keeps_the_serial_prefix(default_detector):
             np.testing.assert_array_equal(off, np.asarray(want["tupleOff"], np.int64)[:32768])
             np.testing.assert_array_equal(np.asarray(got["tupleHits"])[:off[-1]],
                                           np.asarray(want["tupleHits"])[:off[-1]])
+
+
+@pytest.mark.parametrize("room", [-1, 0, 1])
+def test_container_of_about_the_events_own_tuple_count(default_detector, room):
+    """A tuple container one smaller, equal to and one larger than the event's
+    number of tuples: a full one (the first two) ends its last bin where it
+    starts, as the reference's bulkFinalizeFill does, and the event equals the
+    oracle at that capacity in every run."""
+    import oracle
+    import pixgpu
+    caps = {"tuples": 1 << 17, "multiplicity": 1 << 17, "hit_to_tuple": 1 << 20}
+    raw = default_detector.event(20261203 + 7055, 55)  # dense model
+    n = oracle.Oracle(default_detector.es, caps=caps).process(raw)["nTuples"]
+    caps["tuples"] = caps["multiplicity"] = n + room
+    want = oracle.Oracle(default_detector.es, caps=caps).process(raw)
+    assert want["nTuples"] == (n if room > 0 else n + room - 1)
+    ch = pixgpu.Chain(default_detector.es, max_events=1, max_words_per_batch=400000, caps=caps)
+    try:
+        for _ in range(8):
+            ch.process([raw])
+            assert bool(ch.counts(0)["flags"] & pixgpu.PG_FLAG_TUPLE_OVERFLOW) == (room <= 0)
+            diffs = oracle.compare(want, ch.products(0), rtol=RTOL)
+            assert diffs == [], "\n".join("%s: %s" % d for d in diffs)
+    finally:
+        ch.close()
