@@ -688,7 +688,8 @@ __device__ void rfLineFit(const double* H, const float* ge, const RfCircle& circ
     t(0, 1) = m5;
     t(1, 0) = gxz * j3 + gyz * j4;
     t(1, 1) = gzz;
-    szz[i] = sandwich(rot, t)(1, 1);
+    // (J's zeros times an infinite or NaN element of J Cov are NaN)
+    szz[i] = sandwich(rot, t)(1, 1) + 0. * (m0[0] + m0[1] + m0[2] + m3 + m4 + m5 + gzz);
     zz[i] = S(H[3 * i + 2]);
   }
   M<N, N> cms;

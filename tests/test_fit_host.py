@@ -67,6 +67,36 @@ def test_device_broken_line_arithmetic_equals_oracle(host_lib, default_detector,
                 oracle.Oracle(default_detector.es).fit(N, hits, ge))
 
 
+def special_tuples(N):
+    """Tuples with one element of a hit or of its covariance replaced by an
+    infinite, NaN, zero or huge value: 20 of each."""
+    import pixgpu
+    hits, ge, _ = pixgpu.fit_tuples(61 + N, 20, N)
+    hs, gs = [], []
+    with np.errstate(over="ignore"):
+        for value in (np.inf, -np.inf, np.nan, 0.0, 1e20, -1e38):
+            for i in range(N):
+                for k in range(9):
+                    h, g = hits.copy(), ge.copy()
+                    if k < 3:
+                        h[:, i, k] = value
+                    else:
+                        g[:, i, k - 3] = value
+                    hs.append(h)
+                    gs.append(g)
+    return np.concatenate(hs), np.concatenate(gs)
+
+
+@pytest.mark.parametrize("N", [3, 4])
+@pytest.mark.parametrize("algo", ["riemann"])
+def test_device_fit_of_special_values_equals_oracle(host_lib, default_detector, algo, N):
+    """Where a fit's matrices have constant zeros whose products the kernels
+    leave out, an infinite or NaN factor still makes the result NaN."""
+    hits, ge = special_tuples(N)
+    check_equal(host_fit(host_lib, N, hits, ge, False, algo),
+                oracle.Oracle(default_detector.es).fit(N, hits, ge, riemann=algo == "riemann"))
+
+
 @pytest.mark.parametrize("nh,N,index", [(3, 3, 139459), (5, 4, 102442), (5, 4, 126818)])
 def test_mixed_riemann_stays_finite_where_single_precision_cancels(host_lib, nh, N, index):
     """Tuples of the seeded sets of the mixed-precision test whose radial hit
