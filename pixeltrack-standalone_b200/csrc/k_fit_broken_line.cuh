@@ -224,9 +224,10 @@ __device__ void blFit(const double* H3, const float* ge, double B, FitOut& out) 
       const double j1 = lpar[1] * R(0, 1) * j0;
       lpar[1] = lpar[1] * j2;
       lpar[0] = (R(0, 1) + lpar[0] * R(0, 0)) * j2;
-      const double t00 = j0 * lcov(0, 0), t01 = j0 * lcov(0, 1);
+      // (the zero times an infinite or NaN element is NaN)
+      const double t00 = j0 * lcov(0, 0), t01 = j0 * lcov(0, 1) + 0. * lcov(1, 1);
       const double t10 = j1 * lcov(0, 0) + j2 * lcov(1, 0), t11 = j1 * lcov(0, 1) + j2 * lcov(1, 1);
-      lcov(0, 0) = t00 * j0;
+      lcov(0, 0) = t00 * j0 + 0. * t01;
       lcov(0, 1) = t00 * j1 + t01 * j2;
       lcov(1, 0) = t10 * j0;
       lcov(1, 1) = t10 * j1 + t11 * j2;

@@ -88,7 +88,7 @@ def special_tuples(N):
 
 
 @pytest.mark.parametrize("N", [3, 4])
-@pytest.mark.parametrize("algo", ["riemann"])
+@pytest.mark.parametrize("algo", ["broken_line", "riemann"])
 def test_device_fit_of_special_values_equals_oracle(host_lib, default_detector, algo, N):
     """Where a fit's matrices have constant zeros whose products the kernels
     leave out, an infinite or NaN factor still makes the result NaN."""
