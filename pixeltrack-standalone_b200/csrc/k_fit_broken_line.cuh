@@ -311,13 +311,16 @@ __device__ void blFit(const double* H3, const float* ge, double B, FitOut& out) 
     double tmp1 = emdx * emdx + emdy * emdy;
     // The Jacobian (a0 a1 0; 0 0 0; 0 0 q) of (phi, dca, k) by the two offsets
     // and the curvature correction: the reference's elements of dca have the
-    // integer factor q / 2, which is zero (BrokenLine.h, the circle fit's jacobian).
+    // integer factor q / 2, which is zero (BrokenLine.h, the circle fit's
+    // jacobian), over a square root: they are NaN, and so is the covariance,
+    // where the chord is no shorter than the circle's diameter.
+    const double nil = sqr(2 * ff[2]) - tmp1 > 0. ? 0. : NAN;
     const double a0 = (radii[1][0] * emdx - emdy * radii[0][0]) / tmp1;
     const double a1 = (radii[1][1] * emdx - emdy * radii[0][1]) / tmp1;
     const double t00 = a0 * I(0, 0) + a1 * I(1, 0), t01 = a0 * I(0, 1) + a1 * I(1, 1);
     const double t02 = a0 * I(0, n) + a1 * I(1, n);
     const double t20 = q * I(n, 0), t21 = q * I(n, 1), t22 = q * I(n, n);
-    ccov(0, 0) = t00 * a0 + t01 * a1;
+    ccov(0, 0) = t00 * a0 + t01 * a1 + nil;
     ccov(0, 2) = t02 * q;
     ccov(2, 0) = t20 * a0 + t21 * a1;
     // the zeros' terms are left out here too

@@ -335,13 +335,14 @@ __device__ void blFitMixed(const float* H3, const float* ge, double x0, double y
     cpar[1] = double(-q * (quarter / (ff[2] + sqrtf(sqrf(ff[2]) - quarter))));
     cpar[2] = double(q * (1.f / ff[2] + float(u[n])));
     const float tmp1 = emdx * emdx + emdy * emdy;
-    // the Jacobian of blFit, whose elements of dca are zero
+    // the Jacobian of blFit, whose elements of dca are zero or NaN
+    const double nil = sqrf(2 * ff[2]) - tmp1 > 0.f ? 0. : NAN;
     const double a0 = double((radii[1][0] * emdx - emdy * radii[0][0]) / tmp1);
     const double a1 = double((radii[1][1] * emdx - emdy * radii[0][1]) / tmp1);
     const double t00 = a0 * I(0, 0) + a1 * I(1, 0), t01 = a0 * I(0, 1) + a1 * I(1, 1);
     const double t02 = a0 * I(0, n) + a1 * I(1, n);
     const double t20 = q * I(n, 0), t21 = q * I(n, 1), t22 = q * I(n, n);
-    ccov(0, 0) = t00 * a0 + t01 * a1;
+    ccov(0, 0) = t00 * a0 + t01 * a1 + nil;
     ccov(0, 2) = t02 * q;
     ccov(2, 0) = t20 * a0 + t21 * a1;
     ccov(2, 2) = t22 * q + 0. * (I(0, 0) + I(0, 1) + I(1, 1) + I(0, n) + I(1, n));

@@ -97,6 +97,33 @@ def test_device_fit_of_special_values_equals_oracle(host_lib, default_detector, 
                 oracle.Oracle(default_detector.es).fit(N, hits, ge, riemann=algo == "riemann"))
 
 
+def grid_covariances(n, N):
+    ge = np.zeros((n, N, 6), np.float32)
+    ge[:, :, [0, 2, 5]] = 1e-4
+    return ge
+
+
+@pytest.mark.parametrize("N", [3, 4])
+def test_device_broken_line_on_a_small_grid_equals_oracle(host_lib, default_detector, N):
+    """Hits on integer points: equal hits, straight lines, and chords that
+    equal the circle's diameter, where the reference's Jacobian is 0 / 0."""
+    hits = np.random.default_rng(1).integers(-2, 3, (20000, N, 3)).astype(np.float64)
+    ge = grid_covariances(len(hits), N)
+    want = oracle.Oracle(default_detector.es).fit(N, hits, ge)
+    assert (np.isfinite(want["state"]).all(1) & np.isnan(want["cov"][:, 0])).sum() >= 10
+    check_equal(host_fit(host_lib, N, hits, ge, False, "broken_line"), want)
+
+
+@pytest.mark.parametrize("hits", [[[-1, 1, 2], [2, -1, -2], [2, 1, 1]],
+                                  [[1, 1, 1], [-2, 2, 1], [0, 0, 0], [-1, 0, 1]]])
+def test_mixed_broken_line_with_a_chord_of_the_diameter(host_lib, hits):
+    """The covariance of a track whose chord equals the diameter in single
+    precision is NaN as in the FP64 fit, its state finite."""
+    got = host_fit(host_lib, len(hits), np.array([hits], np.float64), grid_covariances(1, len(hits)), True,
+                   "broken_line")
+    assert np.isfinite(got["state"]).all() and np.isnan(got["cov"][0, [0, 1, 2, 5, 6, 9]]).all()
+
+
 @pytest.mark.parametrize("nh,N,index", [(3, 3, 139459), (5, 4, 102442), (5, 4, 126818)])
 def test_mixed_riemann_stays_finite_where_single_precision_cancels(host_lib, nh, N, index):
     """Tuples of the seeded sets of the mixed-precision test whose radial hit
