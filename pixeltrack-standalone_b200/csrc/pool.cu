@@ -324,6 +324,7 @@ int pg_submit_pooled(pg_ctx* c, uint32_t nEvents, const uint32_t* handles, uint3
   int rc = e == cudaSuccess ? PG_OK : cudaFail(c, e, "pool gather");
   if (rc == PG_OK) {
     s.nEvents = nEvents;
+    s.nWords = total;
     s.staged = true;
     rc = launchBatch(c, s);
   }

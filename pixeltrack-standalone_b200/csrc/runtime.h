@@ -46,6 +46,7 @@ struct Slot {
   std::map<uint32_t, uint32_t> probeUsed;      // timed launches inside each captured graph
   uint32_t lastProbeUsed = 0;                  // timed launches of the current batch
   uint32_t nEvents = 0;
+  uint32_t nWords = 0;             // FED words of the current batch (with the device FED scan: their bound)
   bool staged = false;
   SlotState state = SlotState::kFree;
   // formatter errors of the current batch, host-scan mode: event k's are
@@ -56,6 +57,12 @@ struct Slot {
   void* dScan = nullptr;
   uint64_t* hRaw = nullptr;
   uint2* hTab = nullptr;
+};
+
+// A slot's last launched batch.
+struct Launched {
+  Slot* slot = nullptr;
+  uint32_t nWords = 0;
 };
 
 // A pinned buffer that holds one unpacked event on its way into the pool.
@@ -111,6 +118,8 @@ struct pg_ctx {
   std::string err;
   std::mutex errMu;  // guards err: the serving loop's threads report errors concurrently
   std::mutex mu;  // slot bookkeeping (the serving loop's threads share it)
+  std::vector<pixgpu::Launched> launched;  // batches that may be in flight, in launch order, at most one per slot
+  std::mutex launchMu;                     // guards launched
 };
 
 namespace pixgpu {
