@@ -283,8 +283,8 @@ int pg_pool_release(pg_ctx* ctx, uint32_t handle);
 int pg_pool_info(pg_ctx* ctx, uint64_t* cap_words, uint64_t* free_words, uint32_t* live_events);
 int pg_submit_pooled(pg_ctx* ctx, uint32_t n_events, const uint32_t* handles, uint32_t flags, uint32_t* slot);
 
-/* Captures the chain of every batch size 1..max_batch on every slot (graphs are
- * otherwise captured on first use). */
+/* Captures the chain of every batch size 1..max_batch (and grid share, see the
+ * launch-shape tuning) on every slot; graphs are otherwise captured on first use. */
 int pg_prepare(pg_ctx* ctx, uint32_t max_batch);
 
 /* Serving loop with continuous batching over a device-resident pool.  Request i
@@ -334,7 +334,9 @@ int pg_probe_read(pg_ctx* ctx, uint32_t slot, uint32_t max, pg_probe_entry* out,
 /* Launch-shape tuning.  Each tunable kernel loops grid-stride over its
  * event's work; its grid x-extent is the default for the batch size times
  * 2^scale, scale in -3..3 (0: default), kept per batch size (a batch uses the
- * table of its size, else of the largest tuned size below it).  Results do
+ * table of its size, else of the largest tuned size below it).  In a context
+ * with more than twice the reference's doublets (cap_doublets) the grids of a
+ * batch with heavy events are larger by another 2 or 4.  Results do
  * not depend on the scales.  pg_tune_kernel_name(i) names the i-th tunable
  * kernel (NULL past the last); kNbrPool, kTrackCount, kTupleDet and kBLFit are
  * kept for saved tables and scale nothing.  pg_tune_set/pg_tune_load need every slot free

@@ -267,7 +267,7 @@ int stageRawBlocks(pg_ctx* c, Slot& s, uint32_t nEvents, const uint8_t* const* r
   const uint32_t* ids = c->hes.scanFeds.data();
   const uint8_t* fedPtr[4096];
   uint32_t fedSize[4096];
-  uint64_t cursor = 0, batchBound = 0;
+  uint64_t cursor = 0, batchBound = 0, most = 0;
   for (uint32_t k = 0; k < nEvents; ++k) {
     if (fedDirectory(raws[k], sizes[k], fedPtr, fedSize) != PG_OK) return fail(c, PG_ERR_FORMAT, "malformed raw record");
     uint64_t bound = 0;
@@ -282,6 +282,7 @@ int stageRawBlocks(pg_ctx* c, Slot& s, uint32_t nEvents, const uint8_t* const* r
     }
     if (bound > c->caps.fedWords) return fail(c, PG_ERR_CAPACITY, "event or batch too large");
     batchBound += bound;
+    most = std::max(most, bound);
   }
   if (batchBound > c->cfg.max_words_per_batch) return fail(c, PG_ERR_CAPACITY, "event or batch too large");
   cudaError_t e;
@@ -295,6 +296,7 @@ int stageRawBlocks(pg_ctx* c, Slot& s, uint32_t nEvents, const uint8_t* const* r
   s.fmtOff.clear();
   s.nEvents = nEvents;
   s.nWords = uint32_t(batchBound);
+  s.maxWords = uint32_t(most);
   s.staged = true;
   return PG_OK;
 }
@@ -302,7 +304,7 @@ int stageRawBlocks(pg_ctx* c, Slot& s, uint32_t nEvents, const uint8_t* const* r
 int stage(pg_ctx* c, Slot& s, uint32_t nEvents, const uint8_t* const* raws, const size_t* sizes) {
   if (nEvents == 0 || nEvents > c->cfg.max_events) return fail(c, PG_ERR_CAPACITY, "batch size");
   if (s.ws.scan.on) return stageRawBlocks(c, s, nEvents, raws, sizes);
-  uint32_t off = 0;
+  uint32_t off = 0, most = 0;
   const bool fmt = c->cfg.formatter_errors != 0;
   s.fmtErrors.clear();
   s.fmtOff.assign(1, 0);
@@ -316,6 +318,7 @@ int stage(pg_ctx* c, Slot& s, uint32_t nEvents, const uint8_t* const* raws, cons
     s.fmtOff.push_back(uint32_t(s.fmtErrors.size()));
     if (rc != PG_OK) return fail(c, rc, rc == PG_ERR_CAPACITY ? "event or batch too large" : "malformed raw record");
     off += nw;
+    most = std::max(most, nw);
   }
   s.hOffsets[nEvents] = off;
   cudaError_t e;
@@ -331,6 +334,7 @@ int stage(pg_ctx* c, Slot& s, uint32_t nEvents, const uint8_t* const* raws, cons
     return cudaFail(c, e, "H2D offsets");
   s.nEvents = nEvents;
   s.nWords = off;
+  s.maxWords = most;
   s.staged = true;
   return PG_OK;
 }
@@ -346,8 +350,10 @@ int ensureSide(pg_ctx* c, Slot& s) {
   return e == cudaSuccess ? PG_OK : cudaFail(c, e, "side stream");
 }
 
+uint32_t graphKey(uint32_t n, int share) { return n | uint32_t(share) << 16; }
+
 // Captures runChain + result packing for `n` events on the slot's stream.
-int captureGraph(pg_ctx* c, Slot& s, uint32_t n, cudaGraphExec_t* out) {
+int captureGraph(pg_ctx* c, Slot& s, uint32_t n, int share, cudaGraphExec_t* out) {
   const int sr = ensureSide(c, s);
   if (sr != PG_OK) return sr;
   cudaGraph_t g = nullptr;
@@ -357,11 +363,12 @@ int captureGraph(pg_ctx* c, Slot& s, uint32_t n, cudaGraphExec_t* out) {
   if (pr) pr->used = 0;
   tProbe = pr;
   s.ws.tune = tuningFor(c, n);
+  s.ws.tune.share = int8_t(share);
   cudaError_t le =
       runChain(c->des, s.ws, n, s.stream, s.side, s.dRes, c->cfg.riemann_fit != 0, int(c->cfg.vertex_algo));
   if (le == cudaSuccess) le = cudaGetLastError();
   tProbe = nullptr;
-  s.probeUsed[n] = pr ? pr->used : 0;
+  s.probeUsed[graphKey(n, share)] = pr ? pr->used : 0;
   e = cudaStreamEndCapture(s.stream, &g);
   if (le != cudaSuccess || e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
@@ -388,13 +395,36 @@ int copyOut(pg_ctx* c, Slot& s, const T* src, size_t n, void* dst, size_t cap, s
 
 }  // namespace
 
-int pixgpu::captureGraphFor(pg_ctx* c, Slot& s, uint32_t n) {
-  if (s.graphs.count(n)) return PG_OK;
+int pixgpu::captureGraphFor(pg_ctx* c, Slot& s, uint32_t n, int share) {
+  if (s.graphs.count(graphKey(n, share))) return PG_OK;
   cudaGraphExec_t g = nullptr;
-  int rc = captureGraph(c, s, n, &g);
+  int rc = captureGraph(c, s, n, share, &g);
   if (rc != PG_OK) return rc;
-  s.graphs.emplace(n, g);
+  s.graphs.emplace(graphKey(n, share), g);
   return PG_OK;
+}
+
+int pixgpu::maxGridShare(const pg_ctx* c) { return c->caps.cells > 2 * uint32_t(PF_MAX_DOUBLETS_PARAM) ? 2 : 0; }
+
+// Log2 of the larger grid share that each event of the slot's batch gets in a
+// context with raised doublet capacity (tunedGrid).  A batch of heavy events
+// ends with the heaviest, whose share of the grid is what runs then; for
+// lighter ones the larger grids only cost their idle blocks.  By the words of
+// the heaviest event, events/s at share 1 / 2 / 4, one batch and three in flight:
+//   PU65 (73k), 4 events        5255 5162 4958    9792  9179  8533
+//   PU20-75 (84k), 12          11981 11980 11540  18262 17325 16342
+//   PU20-100 (113k), 12         8595 9021 8823   12889 12554 11977
+//   PU100 (113k), 2             2177 2203 2154    4303  4220  4078
+//   PU20-150 (169k), 12         4558 5075 5129    6610  6694  6494
+//   PU20-200 (225k), 12         2470 2762 2861    3689  3769  3737
+//   PU100-200 (225k), 12        1860 1991 2027    2463  2489  2441
+//   PU150 (169k), 12            2210 2293 2301    2670  2666  2597
+// so the lines lie between 84k and 113k words, and, where the heaviest event
+// stands out from the others, between 113k and 169k.
+static int gridShare(const pg_ctx* c, const Slot& s) {
+  if (maxGridShare(c) == 0 || s.maxWords < 95000) return 0;
+  const bool standsOut = 4ull * s.nEvents * s.maxWords > 5ull * s.nWords;
+  return s.maxWords >= 140000 && standsOut ? 2 : 1;
 }
 
 // Batches that run side by side: any number while their FED words stay within
@@ -432,11 +462,13 @@ static void forgetLaunch(pg_ctx* c, const Slot& s) {
 int pixgpu::launchBatch(pg_ctx* c, Slot& s) {
   cudaError_t e;
   if (c->cfg.use_graphs) {
-    int rc = captureGraphFor(c, s, s.nEvents);
+    const int share = gridShare(c, s);
+    int rc = captureGraphFor(c, s, s.nEvents, share);
     if (rc != PG_OK) return rc;
     if ((e = waitForRoom(c, s)) != cudaSuccess) return cudaFail(c, e, "batch order");
-    s.lastProbeUsed = s.probeUsed[s.nEvents];
-    e = cudaGraphLaunch(s.graphs[s.nEvents], s.stream);
+    const uint32_t key = graphKey(s.nEvents, share);
+    s.lastProbeUsed = s.probeUsed[key];
+    e = cudaGraphLaunch(s.graphs[key], s.stream);
     if (e != cudaSuccess) return cudaFail(c, e, "graph launch");
   } else {
     const int sr = ensureSide(c, s);
@@ -446,6 +478,7 @@ int pixgpu::launchBatch(pg_ctx* c, Slot& s) {
     if (pr) pr->used = 0;
     tProbe = pr;
     s.ws.tune = tuningFor(c, s.nEvents);
+    s.ws.tune.share = int8_t(gridShare(c, s));
     e = runChain(c->des, s.ws, s.nEvents, s.stream, s.side, s.dRes, c->cfg.riemann_fit != 0,
                  int(c->cfg.vertex_algo));
     tProbe = nullptr;

@@ -238,6 +238,7 @@ extern const char* const kTuneNames[kNumTune];
 constexpr int kTuneMinScale = -3, kTuneMaxScale = 3;
 struct LaunchTuning {
   int8_t scale[kNumTune];
+  int8_t share;  // of the batch at hand, not of a table: log2 of the grid shares of heavy events (gridShare)
 };
 
 struct Workspace {
@@ -417,16 +418,17 @@ cudaError_t runCleaners(Workspace& ws, uint32_t nEvents, cudaStream_t stream);
 
 // batch input descriptor and compact results (k_pack.cu)
 void launchSetInput(Workspace& ws, const uint32_t* words, const uint8_t* fedIds, cudaStream_t s);
-// Grid x-extent of a tunable launch.  Contexts whose doublet capacity is
-// raised serve events of very different sizes (the tables are tuned at PU50):
-// a batch ends with its heaviest events, whose share of the grid is what runs
-// then, so the shares are larger there (12 uneven PU20-200 events: kConnect
-// -141 us, kFishbone -108 us, the other CA kernels about -40 us each at four
-// times the grid; the doublet kernels, whose staging shares shrink with it,
-// gain at twice: -56 and -42 us).
+// Grid x-extent of a tunable launch: the table's scale (tuned at PU50), and a
+// larger share for each event of a batch of heavy ones (gridShare).  The
+// doublet kernels, whose staging shares shrink with it, take twice at most; the
+// flat grids over the whole batch and the two scatters into CSR lists (12
+// uneven events: kTrackFill 139 -> 160 us, kEdgeScatter 198 -> 210 us at four
+// times) stay as they are.
 inline uint32_t tunedGrid(const Workspace& ws, TuneId id, uint32_t base) {
-  const bool wide = ws.cap.cells > 2 * uint32_t(PF_MAX_DOUBLETS_PARAM);
-  const int s = ws.tune.scale[id] + (!wide ? 0 : id == kTuneDoubletCount || id == kTuneDoubletWrite ? 1 : 2);
+  const bool flat = id == kTuneRawToDigi || id == kTuneModuleBoundaries;
+  const bool scatter = id == kTuneTrackFill || id == kTuneEdgeScatter;
+  const int most = flat || scatter ? 0 : id == kTuneDoubletCount || id == kTuneDoubletWrite ? 1 : 2;
+  const int s = ws.tune.scale[id] + (ws.tune.share < most ? ws.tune.share : most);
   const uint64_t g = s >= 0 ? uint64_t(base) << s : uint64_t(base) >> (-s);
   return uint32_t(g < 1 ? 1 : (g > 65535 ? 65535 : g));
 }

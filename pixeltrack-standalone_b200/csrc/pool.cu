@@ -278,7 +278,7 @@ int pg_submit_pooled(pg_ctx* c, uint32_t nEvents, const uint32_t* handles, uint3
     c->slots[k].state = SlotState::kBusy;
   }
   Slot& s = c->slots[k];
-  uint32_t total = 0, lastH = handles[0];
+  uint32_t total = 0, most = 0, lastH = handles[0];
   cudaEvent_t lastUpload = nullptr;
   {
     std::lock_guard<std::mutex> lk(p.mu);
@@ -295,6 +295,7 @@ int pg_submit_pooled(pg_ctx* c, uint32_t nEvents, const uint32_t* handles, uint3
       const PoolEntry& en = p.entries[h];
       s.hRefs[i] = PoolRef{en.start, en.nWords, total, 0};
       total += en.nWords;
+      most = std::max(most, en.nWords);
       if (en.seq > p.entries[lastH].seq) lastH = h;
     }
     if (!bad && total > c->cfg.max_words_per_batch) bad = 2;
@@ -325,6 +326,7 @@ int pg_submit_pooled(pg_ctx* c, uint32_t nEvents, const uint32_t* handles, uint3
   if (rc == PG_OK) {
     s.nEvents = nEvents;
     s.nWords = total;
+    s.maxWords = most;
     s.staged = true;
     rc = launchBatch(c, s);
   }

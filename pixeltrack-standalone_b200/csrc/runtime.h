@@ -40,13 +40,14 @@ struct Slot {
   PoolRef* dRefs = nullptr;        // device
   uint8_t* hRes = nullptr;         // mapped pinned result region [maxEvents][kResultStride]
   uint8_t* dRes = nullptr;         // its device alias
-  std::map<uint32_t, cudaGraphExec_t> graphs;  // captured chain per batch size
+  std::map<uint32_t, cudaGraphExec_t> graphs;  // captured chain per batch size and grid share (graphKey)
   std::vector<uint32_t> poolHandles;           // pool entries gathered by the current batch
   KernelProbe* probe = nullptr;                // kernel timing events (when a probe is set)
-  std::map<uint32_t, uint32_t> probeUsed;      // timed launches inside each captured graph
+  std::map<uint32_t, uint32_t> probeUsed;      // timed launches inside each captured graph (same key)
   uint32_t lastProbeUsed = 0;                  // timed launches of the current batch
   uint32_t nEvents = 0;
   uint32_t nWords = 0;             // FED words of the current batch (with the device FED scan: their bound)
+  uint32_t maxWords = 0;           // of its largest event
   bool staged = false;
   SlotState state = SlotState::kFree;
   // formatter errors of the current batch, host-scan mode: event k's are
@@ -139,8 +140,10 @@ int unpackRaw(const std::vector<uint32_t>& fedIds, const uint8_t* raw, size_t n,
               uint32_t cap, uint32_t* nWordsOut, std::vector<PfFormatterError>* fmt = nullptr);
 // chain + result packing for the slot's current batch (graph or plain launches)
 int launchBatch(pg_ctx* c, Slot& s);
-// captures the chain for n events on slot s once (no-op when present)
-int captureGraphFor(pg_ctx* c, Slot& s, uint32_t n);
+// the largest log2 grid share of a context's batches (gridShare)
+int maxGridShare(const pg_ctx* c);
+// captures the chain for n events at a grid share on slot s once (no-op when present)
+int captureGraphFor(pg_ctx* c, Slot& s, uint32_t n, int share);
 // a free slot index, or -1
 int findFreeSlot(pg_ctx* c);
 // pool set-up / teardown and reclamation of extents whose gather has finished

@@ -24,7 +24,8 @@ namespace pixgpu {
 int poolStage(pg_ctx* c, const uint8_t* raw, size_t size, uint32_t* stager, uint32_t* nWords);
 int poolCommit(pg_ctx* c, uint32_t stager, uint32_t nWords, uint32_t* handle);
 void poolUnstage(pg_ctx* c, uint32_t stager);
-int captureGraphFor(pg_ctx* c, Slot& s, uint32_t n);
+int maxGridShare(const pg_ctx* c);
+int captureGraphFor(pg_ctx* c, Slot& s, uint32_t n, int share);
 }  // namespace pixgpu
 
 using namespace pixgpu;
@@ -66,10 +67,11 @@ int pg_prepare(pg_ctx* c, uint32_t maxBatch) {
   cudaSetDevice(c->cfg.device);
   maxBatch = std::min(maxBatch ? maxBatch : c->cfg.max_events, c->cfg.max_events);
   for (auto& s : c->slots)
-    for (uint32_t n = 1; n <= maxBatch; ++n) {
-      int rc = captureGraphFor(c, s, n);
-      if (rc != PG_OK) return rc;
-    }
+    for (uint32_t n = 1; n <= maxBatch; ++n)
+      for (int share = 0; share <= maxGridShare(c); ++share) {
+        int rc = captureGraphFor(c, s, n, share);
+        if (rc != PG_OK) return rc;
+      }
   return PG_OK;
 }
 

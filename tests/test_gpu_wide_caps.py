@@ -107,3 +107,28 @@ def test_container_of_about_the_events_own_tuple_count(default_detector, room):
             assert diffs == [], "\n".join("%s: %s" % d for d in diffs)
     finally:
         ch.close()
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_grid_shares_do_not_change_results(default_detector, graphs):
+    """The grids follow the batch's heaviest event: batches below, between and
+    above the lines of that rule, in turn on one slot, give every event its own
+    result."""
+    import pixgpu
+    pus = [20, 60, 110, 170]
+    raws = [default_detector.event(510 + k, pu, model="calibrated") for k, pu in enumerate(pus)]
+    ch = pixgpu.Chain(default_detector.es, max_events=3, max_words_per_batch=3 * 400000, caps=pixgpu.WIDE_CAPS,
+                      use_graphs=graphs)
+    names = ("cellInner", "cellOuter", "tupleOff", "tupleHits", "quality", "state", "cov", "chi2", "zv", "sortInd", "idv")
+    try:
+        alone = []
+        for r in raws:
+            ch.process([r])
+            alone.append({k: ch.product(0, k).tobytes() for k in names})
+        for batch in ([0, 1], [2, 2, 2], [0, 1, 3], [1, 0], [2, 0], [3, 3, 3], [0, 1, 3]):
+            ch.process([raws[k] for k in batch])
+            for e, k in enumerate(batch):
+                assert ch.counts(e)["flags"] == 0
+                assert {n: ch.product(e, n).tobytes() for n in names} == alone[k], (batch, e)
+    finally:
+        ch.close()
