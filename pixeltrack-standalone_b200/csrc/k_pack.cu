@@ -51,7 +51,7 @@ __device__ __forceinline__ uint32_t packHalves(uint32_t w, uint32_t n, F&& get) 
 // reached over the bus: every array is written as consecutive 32-bit words
 // by consecutive threads (whole lines per warp), from all the cluster's SMs
 // at once; the gathers come from device memory.
-constexpr uint32_t kPackCtas = 8;  // CTAs per event in a small batch
+constexpr uint32_t kPackCtas = 2;  // CTAs per event in a small batch
 
 // dynamic shared memory: the slice's loose tuple indices and the whole list
 constexpr size_t kPackSmemBytes = 2 * size_t(kResultTracks) * sizeof(uint32_t);
@@ -235,14 +235,19 @@ cudaError_t runVerticesAndPack(Workspace& ws, uint32_t nEvents, int vertexAlgo, 
   }
   // The track packing is bound by the bus to the host and the vertex finder by
   // the chain of its steps on a few SMs: side by side they take the longer of
-  // the two times (one PU50 event: 24 and 50 us, 64 of them: 300 and 90 us).
+  // the two times (64 PU50 events: 262 and 90 us).
   if ((e = cudaEventRecord(side.fork, stream)) != cudaSuccess) return e;
   if ((e = cudaStreamWaitEvent(side.stream, side.fork, 0)) != cudaSuccess) return e;
   // The vertex finder goes first: its clusters need whole SMs of one GPC, and
   // waited for the packing's CTAs where those came first (8 PU50 events: 69 -> 80 us).
   const cudaError_t ev = runVertices(ws, nEvents, stream, vertexAlgo);
-  // four CTAs per event keep the bus busy once there are a few events
-  const uint32_t P = nEvents <= 4 ? kPackCtas : (nEvents <= kClusterMaxEvents ? kPackCtas / 2 : 1);
+  // Two CTAs per event in a small batch: beside the vertex finder more of them
+  // only take its SMs, and one is too slow for a heavy event.  Events/s at 8 /
+  // 4 / 2 / 1 CTAs: 16 PU50 events 14618 14640 14779 14742 (three batches in
+  // flight 19661 19798 20049 20329), 4 PU50 events 6405 6387 6426 6422, one PU200
+  // event 461 461 461 443, 12 PU20-200 events 2892 2893 2888 2795.  Above 16
+  // events one each, as the bus is busy then.
+  const uint32_t P = nEvents <= kClusterMaxEvents ? kPackCtas : 1;
   PG_PROBED("kPackTracks", side.stream,
             e = launchClustered(kPackTracks, P, nEvents, 512, kPackSmemBytes, side.stream, ws, out));
   // the side stream is joined whatever fails, so that a capture ends cleanly
