@@ -43,3 +43,25 @@ def test_fit_of_any_number_of_tuples(default_detector, entry, N):
             assert np.array_equal(got[k][:n], want[k][:n]), (n, k)
             assert (got[k][n:] == sentinel).all(), (n, k)
     chain.close()
+
+
+@pytest.mark.parametrize("entry,block", [("pg_fit_broken_line", 256), ("pg_fit_broken_line_mixed", 256),
+                                         ("pg_fit_riemann", 128), ("pg_fit_riemann_mixed", 128)])
+@pytest.mark.parametrize("N", [3, 4])
+def test_fit_of_more_tuples_than_one_pass_of_the_grid(default_detector, entry, block, N):
+    """The grid has at most 16 blocks per SM: with one block's tuples and a
+    ragged warp more than that, the first blocks take a second tile, into the
+    shared memory that still held the first one's results."""
+    import pixgpu
+    chain = pixgpu.Chain(default_detector.es, max_events=1, max_words_per_batch=300000)
+    one = 148 * 16 * block
+    n, some = one + block + 33, 4 * block
+    base, ge, _ = pixgpu.fit_tuples(199 + N, some, N)
+    times = n // some + 1  # the same tuples over and over: every repetition has the same results
+    got = _fit(chain, entry, N, np.tile(base, (times, 1, 1)), np.tile(ge, (times, 1, 1)), n)
+    want = _fit(chain, entry, N, base, ge, some)
+    sentinel = np.float32(-77.0).view(np.uint32)
+    for k in SIZES:
+        assert np.array_equal(got[k][:n], np.tile(want[k][:some], (times, 1))[:n]), k
+        assert (got[k][n:] == sentinel).all(), k
+    chain.close()
