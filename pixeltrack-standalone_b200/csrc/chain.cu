@@ -121,7 +121,7 @@ void layout(Workspace& ws, Carver& c, uint32_t E, uint32_t W, const Caps& cap) {
   c.take(ws.scanState, size_t(E) * kScanCalls * ws.scanTiles);
   c.take(ws.scanTicket, size_t(E) * kScanCalls);
   c.take(ws.scanEpoch, E);
-  c.take(ws.bigSeg, size_t(E) * kBigSegCap);
+  c.take(ws.bigMod, size_t(E) * kModStride);
   c.take(ws.segList, size_t(E) * cap.cells);
 }
 

@@ -1148,8 +1148,8 @@ __global__ void kNtupletWrite(Workspace ws) {
 __device__ __forceinline__ uint32_t tupleSize(const uint32_t* toff, uint32_t t) { return toff[t + 1] - toff[t]; }
 
 // cells of stored tuple t, from its cell slots: unlike tupleSize this also
-// holds for the last bin of a full container, whose size the finalize sets to
-// zero after the tuple was written and added to its cells' track lists
+// holds for the last bin of a full container, which ends where it starts
+// although its tuple is written and in its cells' track lists (kNtupletWrite)
 __device__ __forceinline__ uint32_t tupleCellCount(const uint32_t* tcell, uint32_t t) {
   uint32_t n = 0;
   while (n < 4 && tcell[4 * t + n] != 0xffffffffu) ++n;
@@ -1234,17 +1234,18 @@ __global__ void kEarlyDup(Workspace ws) {
   }
 }
 
-// TupleMultiplicity: counts per hit multiplicity, then fill (order irrelevant to the fits)
-// TupleMultiplicity (countMultiplicity/fillMultiplicity, Impl.h:304-338):
-// one block per event counts the non-duplicate tuples of 3, 4 and 5 hits,
-// places the bins, and fills them in ascending tuple order (the serial fill
-// order) with one scan of the three counters packed into 64 bits, so that
-// the content stays deterministic when a bin overflows.
 constexpr uint32_t kMultiplicityCtas = 8;  // in a small batch; pairs in a large one
-// A cluster of P CTAs per event splits the tuples (CTA r takes the r-th part,
-// its counts read by the others through distributed shared memory), since
-// one CTA's two walks are bound by the latency of its loads: 12 uneven events
-// (PU 20-200) took 427 us, all of it the heaviest event's.
+// TupleMultiplicity (countMultiplicity/fillMultiplicity, Impl.h:304-338):
+// counts the non-duplicate tuples of 3, 4 and 5 hits, places the bins, and
+// fills them in ascending tuple order (the serial fill order) with one scan of
+// the three counters packed into 64 bits, so that the content stays
+// deterministic when a bin overflows.  A cluster of P CTAs per event splits the
+// tuples (CTA r takes the r-th part, its counts read by the others through
+// distributed shared memory), since one CTA's two walks are bound by the
+// latency of its loads: 12 uneven events (PU 20-200) took 427 us, all of it the
+// heaviest event's.  Above 16 events pairs: 4 or 8 CTAs made no difference at
+// 24 and 64 PU50 events alone, and cost 0.5 to 1 % with three batches of 64 in
+// flight.
 __global__ void __launch_bounds__(1024) kMultiplicity(Workspace ws) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -1677,7 +1678,7 @@ cudaError_t runCA(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStrea
   // ---- isOuterHitOfCell: scan of the per-hit counts, unordered fill, order per hit
   segScan(ws, kScanOuterHits, ws.ohCount, ws.ohOff, kHitCap + 1, EVF(nHits), kHitCap, nullptr, 0, nEvents, stream, true);
   PG_PROBED("kOuterHitFill", stream, kOuterHitFill<<<dim3(tunedGrid(ws, kTuneOuterHitFill, gx), nEvents), 256, 0, stream>>>(ws));
-  sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.ohCells, kCellCap, ws.ohOff, kHitCap + 1, EVF(nHits), 0, false, kCellCap, 0);
+  sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.ohCells, kCellCap, ws.ohOff, kHitCap + 1, false, kCellCap, 0);
   PG_PROBED("kOhRec", stream, kOhRec<<<dim3(tunedGrid(ws, kTuneOhRec, gx), nEvents), 256, 0, stream>>>(ws));
   // ---- CA links: edges appended unordered, then CSR by inner cell, ordered ascending
   PG_PROBED("kConnect", stream, kConnect<<<dim3(tunedGrid(ws, kTuneConnect, gx * 4), nEvents), kConnectWarps * 32, 0, stream>>>(ws, ws.scratchA, ws.scratchB));
@@ -1685,12 +1686,12 @@ cudaError_t runCA(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStrea
   segScanList(ws, kScanNeighbours, ws.nbrCount, ws.nbrOff, kScanLinked, ws.candidates, &ws.ev[0].nLinked, kCellCap + 1,
               kCellCap, EVF(nCells), kCellCap, sizeof(EventCounters) / 4, nEvents, stream);
   PG_PROBED("kEdgeScatter", stream, kEdgeScatter<<<dim3(tunedGrid(ws, kTuneEdgeScatter, gx), nEvents), 256, 0, stream>>>(ws, ws.scratchA, ws.scratchB));
-  sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.nbr, ws.cap.edges, ws.nbrOff, kCellCap + 1, EVF(nCells), 0, false,
+  sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.nbr, ws.cap.edges, ws.nbrOff, kCellCap + 1, false,
                          min(ws.cap.edges, ws.cap.scratch), 1);
   // ---- early fishbone
   if (ws.ca.earlyFishbone)
     PG_PROBED("kFishbone", stream, kFishbone<<<dim3(tunedGrid(ws, kTuneFishbone, gx * 2), nEvents), 256, 0, stream>>>(ws, false));
-  // ---- n-tuplets: DFS count, scans, DFS write, finalize
+  // ---- n-tuplets: DFS count, scans, write
   PG_PROBED("kNtupletCount", stream, kNtupletCount<<<dim3(tunedGrid(ws, kTuneNtupletCount, gx * 8), nEvents), 128, 0, stream>>>(ws));
   segScan2(ws, kScanStartTuples, ws.startTupleCount, ws.startTupleOff, &ws.ev[0].apcM, kScanStartHits, ws.startHitCount,
            ws.startHitOff, &ws.ev[0].apcN, kCellCap + 1, EVF(nLinked), kCellCap, sizeof(EventCounters) / 4, nEvents,
@@ -1700,7 +1701,7 @@ cudaError_t runCA(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStrea
   segScan(ws, kScanCellTracks, ws.trkCount, ws.trkOff, kCellCap + 1, EVF(nCells), kCellCap, nullptr, 0, nEvents, stream,
           true);
   PG_PROBED("kTrackFill", stream, kTrackFill<<<dim3(tunedGrid(ws, kTuneTrackFill, gx), nEvents), 256, 0, stream>>>(ws));
-  sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.trk, kTupleCellCap, ws.trkOff, kCellCap + 1, EVF(nCells), 0, false, kTupleCellCap, 2);
+  sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.trk, kTupleCellCap, ws.trkOff, kCellCap + 1, false, kTupleCellCap, 2);
   uint32_t* candFlag = ws.startTupleCount;  // scratch
   PG_PROBED("kTrackPool", stream, kTrackPool<<<dim3(tunedGrid(ws, kTuneTrackPool, gx), nEvents), 256, 0, stream>>>(ws, candFlag));
   PG_PROBED("kEarlyDup", stream, kEarlyDup<<<dim3(tunedGrid(ws, kTuneEarlyDup, gx), nEvents), 256, 0, stream>>>(ws));
@@ -1728,7 +1729,9 @@ cudaError_t runCleaners(Workspace& ws, uint32_t nEvents, cudaStream_t stream) {
   uint32_t* indeg = ws.scratchA;        // [maxEvents][cap.scratch], cap.cells per event used
   uint32_t* lists = ws.scratchB;        // two worklists of cap.cells per event (cap.scratch >= 2 cap.cells)
   PG_PROBED("kFastDupInDegree", stream, kFastDupInDegree<<<dim3(tunedGrid(ws, kTuneFastDupInDegree, gx), nEvents), 256, 0, stream>>>(ws, indeg, candFlag));
-  // 24 dense events: 148 us in pairs, 116 us on four CTAs each; 64 PU50 events: 108 us in pairs, 116 us on four
+  // 24 dense events: 148 us in pairs, 116 us on four CTAs each; 64 PU50 events: 108 us in pairs, 116 us on four.
+  // From 17 to 32 events four CTAs make a batch alone 0.6 to 1 % faster at PU20 and PU50 (17, 24, 32 events) and
+  // 24 uneven PU20-200 events 6.6 %; with three batches in flight they cost 0.8 to 1.1 % at PU50 and gain 0.9 % at PU20.
   const uint32_t P = nEvents <= kClusterMaxEvents ? kFastDupCtas : (nEvents <= 2 * kClusterMaxEvents ? 4u : 2u);
   cudaError_t le = cudaSuccess;
   PG_PROBED("kFastDupRounds", stream,
@@ -1738,7 +1741,7 @@ cudaError_t runCleaners(Workspace& ws, uint32_t nEvents, cudaStream_t stream) {
   PG_PROBED("kHitToTupleCount", stream, kHitToTupleCount<<<dim3(tunedGrid(ws, kTuneHitToTupleCount, gx), nEvents), 256, 0, stream>>>(ws));
   segScan(ws, kScanHitTuples, ws.h2tCount, ws.h2tOff, kHitCap + 1, EVF(nHits), kHitCap, nullptr, 0, nEvents, stream, true);
   PG_PROBED("kHitToTupleFill", stream, kHitToTupleFill<<<dim3(tunedGrid(ws, kTuneHitToTupleFill, gx), nEvents), 256, 0, stream>>>(ws));
-  sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.h2t, ws.cap.h2t, ws.h2tOff, kHitCap + 1, nullptr, 0, kHitCap, true,
+  sortSegments<uint32_t>(ws, nEvents, stream, gx * 2, ws.h2t, ws.cap.h2t, ws.h2tOff, kHitCap + 1, true,
                          ws.cap.h2t, 3);
   PG_PROBED("kTripletCleaner", stream, kTripletCleaner<<<dim3(tunedGrid(ws, kTuneTripletCleaner, gx * 2), nEvents), 256, 0, stream>>>(ws));
   return cudaGetLastError();

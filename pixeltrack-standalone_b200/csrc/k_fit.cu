@@ -330,12 +330,16 @@ cudaError_t runFits(const DeviceES& es, Workspace& ws, uint32_t nEvents, cudaStr
   const uint32_t gx = nEvents >= 32 ? 8 : (nEvents >= 8 ? 32 : 148);
   dim3 g(gx, nEvents);
   PG_PROBED("kFitZero", stream, kFitZero<<<dim3(tunedGrid(ws, kTuneFitZero, g.x), nEvents), 256, 0, stream>>>(ws));
-  // one wave of blocks of 512 threads per SM; a few events' tuples (a PU50 event
-  // has 10.6k) go in tiles of 64, over all SMs.  The launch table does not scale
-  // this grid: it follows from the SMs alone.
-  // Otherwise tiles of 128: the hits' gathers make the block wait, and two more
-  // blocks per SM fill that better than one wide block in step (64 PU50 events:
-  // 174 us with 256, 167 us with 128).
+  // One wave of blocks, 512 threads on each of the 148 SMs of a B200.  Tiles of
+  // 128: the hits' gathers make the block wait, and two more blocks per SM fill
+  // that better than one wide block in step (64 PU50 events: 174 us with 256, 167
+  // us with 128; the grid before, sized for such events, took 159 us there but
+  // 1035 instead of 480 us on 12 uneven ones).  A few events' tuples (a PU50 event
+  // has 10.6k) go in tiles of 64, over all SMs: one event 0.2 % faster, 2 to 8
+  // events the same with either, 16 events and three batches in flight 1.6 %
+  // slower.  The launch table does not scale this grid: half or a quarter of it
+  // is 1.5 and 4 % slower at 8 events alone, 2 and 6 % at 64 (1 % faster there
+  // with three batches in flight), twice of it changes nothing.
   const uint32_t most = riemann ? kRiemannBlock : kFitBlock;
   const uint32_t fb = nEvents <= 4 ? 64u : 128u, fg = 148 * (512 / fb);
   static std::atomic<uint64_t> configured[4];

@@ -676,7 +676,7 @@ __device__ void clusterModuleBlock(const Workspace& ws, uint32_t e, uint32_t mod
 __global__ void __launch_bounds__(kClusThreads) kFindClustersBig(Workspace ws) {
   const uint32_t e = blockIdx.y;
   const uint32_t n = min(ws.ev[e].nBigMod, kMaxModules);
-  const uint32_t* list = ws.bigSeg + size_t(e) * kBigSegCap;
+  const uint32_t* list = ws.bigMod + size_t(e) * kModStride;
   for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) clusterModuleBlock(ws, e, list[k]);
 }
 
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 7) kFindClustersSmall(Worksp
   if (np > kSmallPix) {
     if (lane == 0) {
       const uint32_t k = atomicAdd(&c->nBigMod, 1u);
-      if (k < kMaxModules) ws.bigSeg[size_t(e) * kBigSegCap + k] = module;
+      if (k < kMaxModules) ws.bigMod[size_t(e) * kModStride + k] = module;
     }
     return;
   }
@@ -1076,7 +1076,7 @@ __device__ void hitsModuleBlock(const DeviceES& es, const Workspace& ws, uint32_
 __global__ void __launch_bounds__(kHitThreads) kGetHitsBig(DeviceES es, Workspace ws) {
   const uint32_t e = blockIdx.y;
   const uint32_t n = min(ws.ev[e].nBigHitMod, kMaxModules);
-  const uint32_t* list = ws.bigSeg + size_t(e) * kBigSegCap;
+  const uint32_t* list = ws.bigMod + size_t(e) * kModStride;
   for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) hitsModuleBlock(es, ws, e, list[k]);
 }
 
@@ -1101,7 +1101,7 @@ __global__ void __launch_bounds__(kHitWarps * 32, 6) kGetHitsSmall(DeviceES es, 
   if (nclus > kSmallClus) {
     if (lane == 0) {
       const uint32_t k = atomicAdd(&c->nBigHitMod, 1u);
-      if (k < kMaxModules) ws.bigSeg[size_t(e) * kBigSegCap + k] = module;
+      if (k < kMaxModules) ws.bigMod[size_t(e) * kModStride + k] = module;
     }
     return;
   }

@@ -49,8 +49,7 @@ __device__ __forceinline__ uint32_t packHalves(uint32_t w, uint32_t n, F&& get) 
 // every CTA gathers the whole list into its own shared memory.  Each CTA then
 // writes one slice of every output array.  The destination is host memory
 // reached over the bus: every array is written as consecutive 32-bit words
-// by consecutive threads (whole lines per warp), from all the cluster's SMs
-// at once; the gathers come from device memory.
+// by consecutive threads (whole lines per warp); the gathers come from device memory.
 constexpr uint32_t kPackCtas = 2;  // CTAs per event in a small batch
 
 // dynamic shared memory: the slice's loose tuple indices and the whole list
@@ -164,6 +163,7 @@ __global__ void __launch_bounds__(512) kPackTracks(Workspace ws, uint8_t* out) {
   // codes, the triplet cleaner, has finished)
   if (r == 0 && threadIdx.x == 0) ws.ev[e].nLoose = nLoose;
 }
+// (the place has cap.cells entries, which resolveCaps keeps at PF_MAX_DOUBLETS_PARAM or more)
 static_assert(kResultTracks <= PF_MAX_DOUBLETS_PARAM, "the loose tuples' list fits the candidates' place");
 
 // What the vertex finder adds: the tracks' vertices, the vertices and the header.

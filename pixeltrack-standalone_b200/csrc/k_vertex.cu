@@ -1,7 +1,8 @@
-// Pixel vertexing on B200: one block per event runs loadTracks,
-// clusterTracksByDensity, fitVertices(50), splitVertices(9),
-// fitVertices(5000) and sortByPt2 with the PixelVertexProducerCUDA
-// configuration (minT=2, eps=0.07, errmax=0.01, chi2max=9, ptMin=0.5).
+// Pixel vertexing on B200: a cluster of CTAs per event runs loadTracks and
+// the neighbour searches of clusterTracksByDensity, its first CTA the rest:
+// fitVertices(50), splitVertices(9), fitVertices(5000) and sortByPt2, with the
+// PixelVertexProducerCUDA configuration (minT=2, eps=0.07, errmax=0.01,
+// chi2max=9, ptMin=0.5).
 // Reference: plugin-PixelVertexFinding/gpuVertexFinderImpl.h:10-43,
 // gpuClusterTracksByDensity.h:20-207, gpuFitVertices.h:15-98,
 // gpuSplitVertices.h:15-125, gpuSortByPt2.h:15-55,
@@ -968,8 +969,10 @@ cudaError_t runVertices(Workspace& ws, uint32_t nEvents, cudaStream_t stream, in
   // latency (8 instead of 4: 93k -> 52k cycles for walking the 318k tuples of a
   // PU200 event); large batches: pairs of CTAs (measured at 64 PU50 events:
   // 0.52 -> 0.39 ms per batch and +2 % throughput with three batches in
-  // flight).  The iterative clusterer does its searches on one CTA; there the
-  // others share the loading only.
+  // flight).  Four CTAs from 17 to 32 events: 24 uneven PU20-200 events 2 % faster
+  // than in pairs; 17, 24 and 32 PU50 events, 24 PU20 ones and 24 dense ones with
+  // and without DBSCAN within 0.4 % either way.  The iterative clusterer does its
+  // searches on one CTA; there the others share the loading only.
   const uint32_t P = nEvents <= kClusterMaxEvents ? kVtxCtas : (nEvents <= 2 * kClusterMaxEvents ? 4u : 2u);
   cudaError_t le = cudaSuccess;
   PG_PROBED("kVertices", stream,

@@ -18,7 +18,6 @@ constexpr uint32_t kPhiTot = 10 * PF_PHI_BINS + 1;       // 1281
 constexpr uint32_t kPhiStride = 1288;
 constexpr uint32_t kMaxVtx = PF_MAX_VTX;
 constexpr uint32_t kErrCap = 4096;                       // digi errors kept per event
-constexpr uint32_t kBigSegCap = 8192;                    // long list segments queued per event and sort
 // hit indices are packed with a module index into one 32-bit word of the
 // doublet search's hit records (11 + 21 bits)
 constexpr uint32_t kMaxHitCapLimit = 1u << 21;
@@ -307,7 +306,9 @@ struct Workspace {
   uint32_t* trkCount;        // [maxEvents][cap.cells + 1]
   uint32_t* trkOff;          // [maxEvents][cap.cells + 1]
   uint32_t* trk;             // [maxEvents][cap.tupleCells()]
-  uint32_t* candidates;      // [maxEvents][cap.cells] cells with >= 2 tracks, in no particular order
+  // [maxEvents][cap.cells], three lists in turn: the cells with CA links, ascending (until kTrackPool); the cells
+  // with >= 2 tracks, in no particular order (until the duplicate rounds end); the loose tuples (kPackTracks)
+  uint32_t* candidates;
   // tuple multiplicity
   uint32_t* tmOff;           // [maxEvents][16]
   uint32_t* tmBins;          // [maxEvents][cap.tuples]
@@ -331,7 +332,7 @@ struct Workspace {
   uint32_t* scanTicket;      // [maxEvents][kScanCalls], cleared by kInitEvents
   uint32_t* scanEpoch;       // [maxEvents], advanced by kInitEvents
   uint32_t scanTiles;        // tiles of the longest scanned array
-  uint32_t* bigSeg;          // [maxEvents][kBigSegCap] long segments awaiting the block sort
+  uint32_t* bigMod;          // [maxEvents][kModStride] modules for the block clusterizer, then for the block rechit kernel
   uint32_t* segList;         // [maxEvents][cap.cells] segments with >= 2 entries (the ones to order)
 };
 
@@ -373,9 +374,10 @@ size_t workspaceBytes(uint32_t maxEvents, uint32_t wordCap, const Caps& cap);
 void workspaceCarve(Workspace& ws, void* base, uint32_t maxEvents, uint32_t wordCap, const Caps& cap);
 
 // Batches up to this many events run the per-event cooperative kernels
-// (result packing, duplicate rounds, vertexing) as clusters of several CTAs
-// per event, for latency; larger batches give each event one CTA, which
-// leaves the other SMs to the concurrently running batch.
+// (result packing, multiplicities, duplicate rounds, vertexing) as larger
+// clusters of CTAs per event, for latency; larger batches give each event
+// fewer CTAs (one to four), which leaves the other SMs to the concurrently
+// running batch.
 constexpr uint32_t kClusterMaxEvents = 16;
 
 // Launch of kernel k on a grid of (x, nEvents) CTAs grouped in clusters of x

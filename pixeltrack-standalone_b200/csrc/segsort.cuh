@@ -117,16 +117,11 @@ __global__ void __launch_bounds__(256) kSortListed(T* data, size_t dataStride, c
 }
 
 // Orders segment s = [off[s], off[s+1]) of data for every segment the
-// preceding fill noted in list `slot` (those with >= 2 entries).  lenPtr/fixedLen (the number of
-// segments) are kept for the callers' readability only.
+// preceding fill noted in list `slot` (those with >= 2 entries).
 template <typename T>
 void sortSegments(Workspace& ws, uint32_t nEvents, cudaStream_t stream, uint32_t gx, T* data, size_t dataStride,
-                  const uint32_t* off, size_t offStride, const uint32_t* lenPtr, uint32_t lenStride, uint32_t fixedLen,
-                  bool desc, uint32_t dataCap, int slot) {
+                  const uint32_t* off, size_t offStride, bool desc, uint32_t dataCap, int slot) {
   const uint32_t stride = sizeof(EventCounters) / 4;
-  (void)lenPtr;
-  (void)lenStride;
-  (void)fixedLen;
   PG_PROBED("kSortSegments", stream,
             kSortListed<T><<<dim3(gx, nEvents), 256, 0, stream>>>(data, dataStride, off, offStride, ws.segList,
                                                                   ws.cap.cells, &ws.ev[0].nSegList[slot], stride,

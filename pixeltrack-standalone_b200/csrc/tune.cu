@@ -38,13 +38,6 @@ int tuneIndex(const char* name) {
   return -1;
 }
 
-// the name the probe sees for a tunable launch
-const char* launchedName(const pg_ctx* c, uint32_t id) {
-  if (id == kTuneFit && c->cfg.riemann_fit) return c->cfg.mixed_fit ? "kRiemannFitMixed" : "kRiemannFit";
-  if (id == kTuneFit && c->cfg.mixed_fit) return "kBLFitMixed";
-  return kTuneNames[id];
-}
-
 void dropGraphs(pg_ctx* c) {
   for (auto& s : c->slots) {
     cudaStreamSynchronize(s.stream);
@@ -194,7 +187,7 @@ int pg_autotune(pg_ctx* c, uint32_t n, const uint8_t* const* raws, const size_t*
     if (id == kTuneFedCopy && !c->cfg.fed_scan) continue;
     // names that saved tables hold, of work that other kernels do now
     if (id == kTuneNbrPool || id == kTuneTrackCount || id == kTuneTupleDet || id == kTuneFit) continue;
-    if ((rc = pg_set_probe(c, launchedName(c, id))) != PG_OK) break;
+    if ((rc = pg_set_probe(c, kTuneNames[id])) != PG_OK) break;
     const int start = tuningFor(c, n).scale[id];
     double best = 0;
     if ((rc = pg_tune_set(c, n, kTuneNames[id], start)) != PG_OK || (rc = timeBatches(&best)) != PG_OK) break;
