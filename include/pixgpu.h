@@ -250,7 +250,10 @@ typedef struct pg_result_view {
 /* Asynchronous batches.  pg_submit unpacks, copies and launches on a free slot
  * and returns its index (PG_ERR_BUSY when every slot is in use); pg_query returns
  * PG_OK when the batch has finished and PG_ERR_BUSY while it runs; pg_wait blocks;
- * pg_result gives the view of event k; pg_release makes the slot free again. */
+ * pg_result gives the view of event k; pg_release makes the slot free again.
+ * Batches run side by side, but large ones (together more than six million FED
+ * words) at most three at a time: a further one's stream waits, after the copies
+ * of its inputs, for a batch launched before it. */
 int pg_submit(pg_ctx* ctx, uint32_t n_events, const uint8_t* const* raws, const size_t* raw_sizes,
               uint32_t* slot);
 int pg_query(pg_ctx* ctx, uint32_t slot);
